@@ -494,6 +494,15 @@ size_t khp_inverse_workspace(int64_t batch, int32_t n);
 int khp_inverse(int64_t batch, int32_t n, int32_t precision, void* A, int64_t a_stride, void* Ainv,
                 int64_t inv_stride, int32_t* status, void* workspace, size_t ws_bytes, void* stream);
 
+/*
+ * The same inverse by Gauss-Jordan elimination with partial pivoting (the form the mixed-precision
+ * solve uses: one launch per call up to n = 128 in FP32, two launches per 32 rows otherwise).
+ * Arguments, status and scratch as khp_inverse; A is overwritten with intermediate values and
+ * must not overlap Ainv.
+ */
+int khp_inverse_gj(int64_t batch, int32_t n, int32_t precision, void* A, int64_t a_stride, void* Ainv,
+                   int64_t inv_stride, int32_t* status, void* workspace, size_t ws_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1055,8 +1055,8 @@ int launch_getrs_blocked(int64_t batch, int n, const cplx<T>* A, int64_t lda, in
 
 // A^-1 = U^-1 L^-1 P: the factors, the permutation matrix P written directly, the substitutions.
 template <typename T>
-int launch_inverse_blocked(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Ainv, int64_t ldi,
-                           int64_t bsI, int* piv, int* info, cudaStream_t s) {
+int launch_inverse_lu(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Ainv, int64_t ldi,
+                      int64_t bsI, int* piv, int* info, cudaStream_t s) {
   if (batch <= 0) return KHP_OK;
   int st = launch_getrf_blocked<T>(batch, n, A, lda, bsA, piv, info, s);
   if (st) return st;
@@ -1106,8 +1106,8 @@ int launch_inverse_blocked(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_
   template int launch_getrf_blocked<T>(int64_t, int, cplx<T>*, int64_t, int64_t, int*, int*, cudaStream_t);     \
   template int launch_getrs_blocked<T>(int64_t, int, const cplx<T>*, int64_t, int64_t, const int*, cplx<T>*,    \
                                        int64_t, int64_t, int, cudaStream_t);                                    \
-  template int launch_inverse_blocked<T>(int64_t, int, cplx<T>*, int64_t, int64_t, cplx<T>*, int64_t, int64_t,  \
-                                         int*, int*, cudaStream_t);
+  template int launch_inverse_lu<T>(int64_t, int, cplx<T>*, int64_t, int64_t, cplx<T>*, int64_t, int64_t,  \
+                                    int*, int*, cudaStream_t);
 
 KHP_INSTANTIATE(double)
 KHP_INSTANTIATE(float)
@@ -1150,10 +1150,10 @@ int khp_inverse(int64_t batch, int32_t n, int32_t precision, void* A, int64_t a_
   int* piv = static_cast<int*>(workspace);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (precision == 0)
-    return launch_inverse_blocked<double>(batch, n, static_cast<cplx<double>*>(A), n, a_stride,
-                                          static_cast<cplx<double>*>(Ainv), n, inv_stride, piv, status, s);
-  return launch_inverse_blocked<float>(batch, n, static_cast<cplx<float>*>(A), n, a_stride,
-                                       static_cast<cplx<float>*>(Ainv), n, inv_stride, piv, status, s);
+    return launch_inverse_lu<double>(batch, n, static_cast<cplx<double>*>(A), n, a_stride,
+                                     static_cast<cplx<double>*>(Ainv), n, inv_stride, piv, status, s);
+  return launch_inverse_lu<float>(batch, n, static_cast<cplx<float>*>(A), n, a_stride,
+                                  static_cast<cplx<float>*>(Ainv), n, inv_stride, piv, status, s);
 }
 
 }  // extern "C"

@@ -127,7 +127,7 @@ int khp_scattering_eig(int64_t batch, int32_t ng, const double* S, int64_t s_str
   ET_TRY(cuda_status());
   // Di = S22^-1 (lu keeps the factors for det(S22))
   ET_TRY(launch_copy<double>(batch, h, h, S22, N, s_stride, p.lu, h, hh, s));
-  ET_TRY(launch_inverse_blocked<double>(batch, h, p.lu, h, hh, p.Di, h, hh, p.piv, status, s));
+  ET_TRY(launch_inverse_lu<double>(batch, h, p.lu, h, hh, p.Di, h, hh, p.piv, status, s));
   cd* A = p.A;
   cd* Atl = A;
   cd* Atr = A + h;

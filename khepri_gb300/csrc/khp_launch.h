@@ -58,6 +58,12 @@ template <typename T>
 int launch_getrs_blocked(int64_t batch, int n, const cplx<T>* A, int64_t lda, int64_t bsA, const int* piv, cplx<T>* B,
                          int64_t ldb, int64_t bsB, int m, cudaStream_t s);
 template <typename T>
+int launch_inverse_lu(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Ainv, int64_t ldi,
+                      int64_t bsI, int* piv, int* info, cudaStream_t s);
+
+// Ainv[b] = A[b]^-1 by Gauss-Jordan elimination (A destroyed; Ainv must not overlap A; piv: batch x n
+// ints of scratch): in registers, or by panels, by size (khp_inverse.cu); launch_inverse_lu beyond.
+template <typename T>
 int launch_inverse_blocked(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Ainv, int64_t ldi,
                            int64_t bsI, int* piv, int* info, cudaStream_t s);
 

@@ -422,6 +422,16 @@ __global__ void k_to_double(int64_t count, const cf* __restrict__ in, cd* out) {
     out[e] = mk((double)in[e].re, (double)in[e].im);
 }
 
+// E = I - P in FP32 (P = W Wi, FP64-accurate).  One grid row per problem.
+__global__ void k_inverse_residual(int64_t boff, int n, const cd* __restrict__ P, cf* E) {
+  const int64_t nn = (int64_t)n * n;
+  const int64_t b = boff + blockIdx.y;
+  for (int rc = blockIdx.x * blockDim.x + threadIdx.x; rc < nn; rc += gridDim.x * blockDim.x) {
+    const cd p = P[b * nn + rc];
+    E[b * nn + rc] = mk((float)((rc / n == rc % n ? 1.0 : 0.0) - p.re), (float)-p.im);
+  }
+}
+
 // lam64 = sqrt(mu64), lam32 = round(lam64).  Principal root (alternative.py:173), except that a
 // root within 1e-8 relative of the imaginary axis is taken with Im >= 0: mu on (or rounded
 // across) the negative real axis then gets one branch, so that degenerate propagating pairs
@@ -1353,6 +1363,17 @@ int grad_mixed(const Table& tb, MixedPlan& p, GradPlan& g, const GradArgs& ga, i
     k_stack_sweep_T<<<(unsigned)batch, 256, 0, s>>>(tb, gx, gy, kp, k0, g.RX, g.RXA, g.RRT, g.Y, g.SWT);
     count_launches(1);
     MX_TRY(cuda_status());
+  }
+  // ---- W^-1 to FP32 rounding: Wi += Wi (I - W Wi), the residual FP64-accurate.  The forward solve only
+  //      needs Wi as a factor of its refinement; here its error (condition of W times FP32's) would pass
+  //      into the gradient (the double-float W and V in M64 are not needed any more) ----
+  const int64_t bm = (int64_t)used.size() * batch;
+  if (bm > 0) {
+    MX_EW(k_to_double, bm * nn, bm * nn, p.Wi[0], p.CW64);
+    MX_TRY(ozaki_zgemm(bm, n, n, n, p.W64[0], n, nn, nullptr, p.CW64, n, nn, p.M64, n, nn, p.oz, s));
+    MX_PP(k_inverse_residual, bm, nn, n, p.M64, p.E32);
+    MX_TRY(launch_gemm<float>(bm, n, n, n, one, p.Wi[0], n, nn, p.E32, n, nn, zero, p.Z32, n, nn, s));
+    MX_TRY(launch_axpby<float>(bm, n, n, one, p.Wi[0], n, nn, one, p.Z32, n, nn, p.Wi[0], n, nn, s));
   }
   // ---- per map slot: H^T, QD^T over its layers, then N = W H^T W^-1 and the C-gradient ----
   const cd* Cm = reinterpret_cast<const cd*>(conv);
