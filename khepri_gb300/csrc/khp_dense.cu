@@ -60,11 +60,12 @@ __global__ void __launch_bounds__(kTeamThreads) k_getrs(int n, const cplx<T>* A,
 // the matrix is large enough for it, else one reflector at a time.
 template <typename T>
 __global__ void __launch_bounds__(kTeamThreads, 3) k_gehrd(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
-                                                         int blocked) {
+                                                         int blocked, const int* __restrict__ only) {
   __shared__ TeamShared sh;
   extern __shared__ unsigned char dyn[];
   TeamCta t;
   const int64_t b = blockIdx.x;
+  if (only && !only[b]) return;
   if (blocked)
     team_gehrd_blocked(t, A + b * bsA, lda, n, Z + b * (int64_t)n * n, n, reinterpret_cast<cplx<T>*>(dyn), &sh);
   else
@@ -77,13 +78,15 @@ __global__ void __launch_bounds__(kTeamThreads, 3) k_gehrd(int n, cplx<T>* A, in
 template <typename T>
 __global__ void __launch_bounds__(kTeamThreads) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
                                                               cplx<T>* lam, int64_t bsLam, int* info,
-                                                              unsigned char* logbuf, int64_t log_bytes) {
+                                                              unsigned char* logbuf, int64_t log_bytes,
+                                                              const int* __restrict__ only) {
   __shared__ TeamShared sh;
   __shared__ cplx<T> win[(KHP_HQR_WIN + 2) * (KHP_HQR_WIN + 2)];
   __shared__ cplx<T> rs[KHP_HQR_WIN];
   __shared__ T rc[KHP_HQR_WIN];
   TeamCta t;
   const int64_t b = blockIdx.x;
+  if (only && !only[b]) return;
   cplx<T>* Ab = A + b * bsA;
   cplx<T>* Zb = Z + b * (int64_t)n * n;
   int st;
@@ -197,9 +200,11 @@ __global__ void __launch_bounds__(kLogRows) k_hqr_apply_log(int n, cplx<T>* Z, c
 
 // Scale every column of W to unit 2-norm (thread per column, coalesced along rows).
 template <typename T>
-__global__ void k_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW) {
+__global__ void k_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW,
+                                 const int* __restrict__ only) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < batch * n; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = e / n;
+    if (only && !only[b]) continue;
     const int k = (int)(e % n);
     cplx<T>* w = W + b * bsW + k;
     T s = T(0);
@@ -216,13 +221,15 @@ __global__ void __launch_bounds__(256) k_gemm(int n, int m, int k, cplx<T> alpha
                                               int64_t lda, int64_t bsA, const cplx<T>* __restrict__ B, int64_t ldb,
                                               int64_t bsB, cplx<T> beta, cplx<T>* C, int64_t ldc, int64_t bsC,
                                               int64_t boff, const int* __restrict__ aidx,
-                                              const int* __restrict__ bidx, cplx<T> bshift) {
+                                              const int* __restrict__ bidx, cplx<T> bshift,
+                                              const int* __restrict__ only) {
   constexpr int TM = BM / 16, TN = BN / 16;
   constexpr int LA = BM * BK / 256, LB = BK * BN / 256;  // tile elements loaded per thread
   static_assert(LA * 256 == BM * BK && LB * 256 == BK * BN, "tile loads must split evenly over 256 threads");
   __shared__ cplx<T> As[BK][BM];
   __shared__ cplx<T> Bs[BK][BN];
   const int64_t b = blockIdx.z + boff;
+  if (only && !only[b]) return;
   A += (aidx ? (int64_t)aidx[b] : b) * bsA;
   B += (bidx ? (int64_t)bidx[b] : b) * bsB;
   C += b * bsC;
@@ -796,7 +803,7 @@ int launch_getrs(int64_t batch, int n, const cplx<T>* A, int64_t lda, int64_t bs
 template <typename T>
 int launch_gemm(int64_t batch, int n, int m, int k, cplx<T> alpha, const cplx<T>* A, int64_t lda, int64_t bsA,
                 const cplx<T>* B, int64_t ldb, int64_t bsB, cplx<T> beta, cplx<T>* C, int64_t ldc, int64_t bsC,
-                cudaStream_t s, const int* aidx, const int* bidx, cplx<T> bshift) {
+                cudaStream_t s, const int* aidx, const int* bidx, cplx<T> bshift, const int* only) {
   if (batch <= 0 || n <= 0 || m <= 0) return KHP_OK;
   // 64 x 64 tiles (4 x 4 outputs per thread) once both output dimensions reach 64; 32 x 128
   // (2 x 8) for outputs of at most 32 rows and at least 128 columns (the block rows of the
@@ -809,13 +816,13 @@ int launch_gemm(int64_t batch, int n, int m, int k, cplx<T> alpha, const cplx<T>
     dim3 grid((m + BN - 1) / BN, (n + BM - 1) / BM, nb);
     if (wide)
       k_gemm<T, 32, 128, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
-                                                  aidx, bidx, bshift);
+                                                  aidx, bidx, bshift, only);
     else if (big)
       k_gemm<T, 64, 64, 8><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
-                                                aidx, bidx, bshift);
+                                                aidx, bidx, bshift, only);
     else
       k_gemm<T, 32, 32, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
-                                                 aidx, bidx, bshift);
+                                                 aidx, bidx, bshift, only);
     count_launches(1);
   }
   return cuda_status();
@@ -824,7 +831,7 @@ int launch_gemm(int64_t batch, int n, int m, int k, cplx<T> alpha, const cplx<T>
 template <typename T>
 int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z, cplx<T>* W, int64_t ldw,
                 int64_t bsW, cplx<T>* lam, int64_t bsLam, int* info, cudaStream_t s, void* logbuf,
-                int64_t log_bytes) {
+                int64_t log_bytes, const int* only) {
   if (batch <= 0) return KHP_OK;
   // blocked reduction when panels pay off and their scratch fits in shared memory
   const size_t scratch = sizeof(cplx<T>) * (size_t)gehrd_blocked_scratch(n);
@@ -838,13 +845,14 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   // the blocked reduction keeps full 256-thread teams (its panel updates are parallel work; three
   // teams per SM already cover the SM), whatever team size suits the QR's serial window chase
   const int gthreads = blocked ? kTeamThreads : threads;
-  k_gehrd<T><<<(unsigned)batch, gthreads, smem, s>>>(n, A, lda, bsA, Z, blocked);
+  k_gehrd<T><<<(unsigned)batch, gthreads, smem, s>>>(n, A, lda, bsA, Z, blocked, only);
   // Z through the rotation log when the region holds at least one full sweep per matrix
   unsigned char* lg = nullptr;
-  if (logbuf && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
+  if (logbuf && !only && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
       hqr_log_view<T>(logbuf, log_bytes, n).cap_rot >= n - 1)
     lg = static_cast<unsigned char*>(logbuf);
-  k_geev_schur<T><<<(unsigned)batch, threads, 0, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes);
+  k_geev_schur<T><<<(unsigned)batch, threads, 0, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes,
+                                                       only);
   count_launches(2);
   int st = cuda_status();
   if (st) return st;
@@ -862,10 +870,17 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
     if (st) return st;
   }
   // W = Z X (X unit upper triangular, stored in A) and unit columns
-  st = launch_gemm<T>(batch, n, n, n, mk(T(1)), Z, n, (int64_t)n * n, A, lda, bsA, mk(T(0)), W, ldw, bsW, s);
-  if (st) return st;
+  st = launch_gemm<T>(batch, n, n, n, mk(T(1)), Z, n, (int64_t)n * n, A, lda, bsA, mk(T(0)), W, ldw, bsW, s, nullptr,
+                      nullptr, mk(T(0)), only);
+  return st ? st : launch_normalize_cols<T>(batch, n, W, ldw, bsW, s, only);
+}
+
+template <typename T>
+int launch_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW, cudaStream_t s,
+                          const int* only) {
   const int64_t cols = batch * n;
-  k_normalize_cols<T><<<(unsigned)std::min<int64_t>((cols + 127) / 128, 152 * 16), 128, 0, s>>>(batch, n, W, ldw, bsW);
+  k_normalize_cols<T><<<(unsigned)std::min<int64_t>((cols + 127) / 128, 152 * 16), 128, 0, s>>>(batch, n, W, ldw, bsW,
+                                                                                               only);
   count_launches(1);
   return cuda_status();
 }
@@ -1093,9 +1108,10 @@ int launch_inverse_lu(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA
                                int64_t, int, cudaStream_t);                                                     \
   template int launch_gemm<T>(int64_t, int, int, int, cplx<T>, const cplx<T>*, int64_t, int64_t, const cplx<T>*, \
                               int64_t, int64_t, cplx<T>, cplx<T>*, int64_t, int64_t, cudaStream_t, const int*, \
-                              const int*, cplx<T>);                                                             \
+                              const int*, cplx<T>, const int*);                                                 \
   template int launch_geev<T>(int64_t, int, cplx<T>*, int64_t, int64_t, cplx<T>*, cplx<T>*, int64_t, int64_t,  \
-                              cplx<T>*, int64_t, int*, cudaStream_t, void*, int64_t);                           \
+                              cplx<T>*, int64_t, int*, cudaStream_t, void*, int64_t, const int*);               \
+  template int launch_normalize_cols<T>(int64_t, int, cplx<T>*, int64_t, int64_t, cudaStream_t, const int*);    \
   template int launch_copy<T>(int64_t, int, int, const cplx<T>*, int64_t, int64_t, cplx<T>*, int64_t, int64_t,  \
                               cudaStream_t);                                                                    \
   template int launch_identity<T>(int64_t, int, int, cplx<T>*, int64_t, int64_t, cplx<T>, cudaStream_t);        \

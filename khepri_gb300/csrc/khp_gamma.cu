@@ -57,6 +57,8 @@ struct GammaPlan {
   // modes scratch (reused per map)
   cplx<T> *M, *Z, *CW, *lu;
   int* piv;
+  char* eig;               // scratch of launch_geev_refined
+  size_t eig_bytes;
   std::vector<int*> midx;  // per distinct map: the map index of every problem
   // per layer
   std::vector<cplx<T>*> lu1, lu2;
@@ -86,6 +88,8 @@ GammaPlan<T> plan_gamma(Arena& a, int64_t batch, int nh, int nlayers, const int*
   p.Z = a.take<cplx<T>>(batch * nn);
   p.CW = a.take<cplx<T>>(batch * nn);
   p.lu = a.take<cplx<T>>(batch * nn);
+  p.eig_bytes = nmaps_used > 0 ? geev_refined_workspace(batch, (int)n) : 0;
+  p.eig = a.take<char>(p.eig_bytes);
   p.piv = a.take<int>(batch * n);
   for (int l = 0; l < nlayers; ++l) {
     if (kinds[l] == 1) {
@@ -207,7 +211,7 @@ int solve_gamma(int64_t batch, int px, int py, int nlayers, const int* kinds, co
     } else {
       GT_TRY(launch_assemble_pq<T>(batch, nh, Cm, reinterpret_cast<const cd*>(hx), reinterpret_cast<const cd*>(hy),
                                    p.midx[m], gx, gy, kp, k0, p.M, s));
-      GT_TRY(launch_geev<T>(batch, n, p.M, n, nn, p.Z, p.W[m], n, nn, p.lam[m], n, status, s));
+      GT_TRY(launch_geev_refined(batch, n, p.M, p.W[m], p.lam[m], status, s, p.eig, p.eig_bytes));
       GT_EW(k_sqrt_lam_t<T>, batch * n, batch * n, p.lam[m]);
       cplx<T>* CWt = p.CW;
       cplx<T>* CWb = p.CW + batch * hn;

@@ -19,19 +19,32 @@ int launch_getrs(int64_t batch, int n, const cplx<T>* A, int64_t lda, int64_t bs
                  int64_t ldb, int64_t bsB, int m, cudaStream_t s);
 
 // C = alpha A B + beta C (A n x k, B k x m).  A batch stride of 0 broadcasts one matrix;
-// aidx / bidx (optional, device int[batch]) pick A[aidx[b]] / B[bidx[b]] for problem b.
+// aidx / bidx (optional, device int[batch]) pick A[aidx[b]] / B[bidx[b]] for problem b; only
+// (optional, device int[batch]): problems with only[b] == 0 are left alone.
 template <typename T>
 int launch_gemm(int64_t batch, int n, int m, int k, cplx<T> alpha, const cplx<T>* A, int64_t lda, int64_t bsA,
                 const cplx<T>* B, int64_t ldb, int64_t bsB, cplx<T> beta, cplx<T>* C, int64_t ldc, int64_t bsC,
-                cudaStream_t s, const int* aidx = nullptr, const int* bidx = nullptr, cplx<T> bshift = cplx<T>{});
+                cudaStream_t s, const int* aidx = nullptr, const int* bidx = nullptr, cplx<T> bshift = cplx<T>{},
+                const int* only = nullptr);
 
 // Eigen-decomposition A W = W diag(lam); A destroyed; Z: batch x n x n scratch (ld n).
 // logbuf (optional, log_bytes per matrix, both multiples of 32): scratch for the QR's rotation
-// log, which defers the updates of Z (used when it holds at least one full sweep).
+// log, which defers the updates of Z (used when it holds at least one full sweep, and without
+// `only`).  only (optional, device int[batch]): matrices with only[b] == 0 are left alone.
 template <typename T>
 int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z, cplx<T>* W, int64_t ldw,
                 int64_t bsW, cplx<T>* lam, int64_t bsLam, int* info, cudaStream_t s, void* logbuf = nullptr,
-                int64_t log_bytes = 0);
+                int64_t log_bytes = 0, const int* only = nullptr);
+// Columns of W to unit 2-norm.
+template <typename T>
+int launch_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW, cudaStream_t s,
+                          const int* only = nullptr);
+
+// M W = W diag(lam) in FP64 (M [batch][n][n] destroyed; unit columns): FP32 eigensolver and FP64
+// refinement, the matrices whose residual test fails by the FP64 eigensolver (khp_mixed.cu).
+size_t geev_refined_workspace(int64_t batch, int n);
+int launch_geev_refined(int64_t batch, int n, cplx<double>* M, cplx<double>* W, cplx<double>* lam, int* info,
+                        cudaStream_t s, void* ws, size_t ws_bytes);
 
 // Element-wise helpers on batches of n x m matrices.
 template <typename T>

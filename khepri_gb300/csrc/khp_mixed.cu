@@ -375,37 +375,52 @@ __device__ __forceinline__ bool rt_undefined(const double* kp, double k0, cd eps
 }
 
 // Eigen-residual check after the last refinement step: MW holds M W (FP64-accurate).  A problem
-// whose relative residual max_i |(M W - W diag(mu))_ij| / (max|mu| max_i |W_ij|) exceeds 1e-8 in
-// any column j, or is not finite, gets KHP_BIT_MODES (unless its R and T are undefined).  One CTA
-// per matrix; lanes take consecutive columns, so each row's loads are coalesced.
-__global__ void __launch_bounds__(256) k_eig_check(int n, const cd* __restrict__ MW, const cd* __restrict__ W,
-                                                   const cd* __restrict__ mu, const double* __restrict__ kp,
-                                                   const double* __restrict__ k0, cd epsi, int* stat) {
+// whose relative residual max_i |(M W - W diag(mu))_ij| / (max|mu| max_i |W_ij|) exceeds tol in any
+// column j, or is not finite, gets `bit` (with kp: unless its R and T are undefined).  A CTA takes 32
+// columns of a matrix, its 8 warps every eighth row each (loads coalesced along rows); the magnitudes
+// are compared squared, without a root per element.  Bound by the FP64 pipe (~14 operations per
+// element): one 242 x 242 matrix on 8 SMs instead of one.
+__global__ void __launch_bounds__(256) k_eig_check(int64_t boff, int n, const cd* __restrict__ MW,
+                                                   const cd* __restrict__ W, const cd* __restrict__ mu,
+                                                   const double* __restrict__ kp, const double* __restrict__ k0,
+                                                   cd epsi, double tol, int bit, int* stat) {
   __shared__ TeamShared sh;
+  __shared__ double rs[8][32], wsq[8][32];
   TeamCta t;
-  const int64_t b = blockIdx.x;
-  if (rt_undefined(kp + 4 * b, k0[b], epsi)) return;
+  const int64_t b = boff + blockIdx.y;
+  if (kp && rt_undefined(kp + 4 * b, k0[b], epsi)) return;
   const int64_t nn = (int64_t)n * n;
   const cd* mb = mu + b * n;
   double big = 0.0;
   int bi = 0;
-  for (int i = t.tid(); i < n; i += t.size()) big = fmax(big, cabs(mb[i]));
+  for (int i = t.tid(); i < n; i += t.size()) big = fmax(big, norm2(mb[i]));
   team_argmax(t, big, bi, &sh);
-  double worst = 0.0;
-  for (int j = t.tid(); j < n; j += t.size()) {
-    double r = 0.0, w = 0.0;
+  const int lane = t.tid() & 31, warp = t.tid() >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  double r = 0.0, w = 0.0;
+  bool nan = false;
+  if (j < n) {
     const cd mj = mb[j];
-    for (int i = 0; i < n; ++i) {
+    for (int i = warp; i < n; i += 8) {
       const int64_t e = b * nn + (int64_t)i * n + j;
       const cd wij = W[e];
-      r = fmax(r, cabs(MW[e] - wij * mj));
-      w = fmax(w, cabs(wij));
+      const double d2 = norm2(MW[e] - wij * mj);
+      nan |= !(d2 == d2);
+      r = fmax(r, d2);
+      w = fmax(w, norm2(wij));
     }
-    const double rel = r / (big * w);
-    worst = rel == rel ? fmax(worst, rel) : INFINITY;  // a NaN fails the test
   }
-  team_argmax(t, worst, bi, &sh);
-  if (t.tid() == 0 && !(worst <= 1e-8)) stat[b] |= KHP_BIT_MODES;
+  rs[warp][lane] = nan ? INFINITY : r;
+  wsq[warp][lane] = w;
+  t.sync();
+  if (warp == 0 && j < n) {
+    for (int q = 1; q < 8; ++q) {
+      r = fmax(r, rs[q][lane]);
+      w = fmax(w, wsq[q][lane]);
+    }
+    r = fmax(r, rs[0][lane]);
+    if (!(r <= tol * tol * big * w)) atomicOr(stat + b, bit);
+  }
 }
 
 // W64 += D32 ; W32 = round(W64)
@@ -1333,6 +1348,120 @@ GradPlan plan_grad(Arena& a, int64_t batch, int nh, int L, int64_t nmaps) {
     MX_TRY(cuda_status());                                                                             \
   } while (0)
 
+// Scratch of refine_eigs: all [batch] matrices (FP32 n x n: W32, Wi, Z32, E32, lu32, F32) and vectors.
+struct EigRefine {
+  cf *W32, *Wi, *Z32, *E32, *lu32, *F32;
+  const cf* lam32;
+  cd *MW64, *mu, *mu_next;
+  int *pair, *nearest, *csz, *memb;
+  cf* xc;
+  int *piv, *st;
+  float *tfA, *tfB;
+  int* tferr;
+  OzakiWs oz;
+};
+
+int launch_eig_check(int64_t batch, int n, const cd* MW, const cd* W, const cd* mu, const double* kp, const double* k0,
+                     cd epsi, double tol, int bit, int* stat, cudaStream_t s) {
+  for (int64_t o = 0; o < batch; o += 65535) {
+    const unsigned nb = (unsigned)std::min<int64_t>(batch - o, 65535);
+    k_eig_check<<<dim3((n + 31) / 32, nb), 256, 0, s>>>(o, n, MW, W, mu, kp, k0, epsi, tol, bit, stat);
+    count_launches(1);
+  }
+  return cuda_status();
+}
+
+// Eigenpairs of the FP64 matrices M from an FP32 eigensolver's (r.W32, r.lam32): W64 and r.mu, by
+// kEigSteps steps of R = M W - W mu in FP64, E = W^-1 R (FP32 inverse of the current W, left in r.Wi),
+// mu += diag(E), W += W F.
+int refine_eigs(int64_t bm, int n, const cd* M64, cd* W64, EigRefine& r, cudaStream_t s) {
+  const int64_t nn = (int64_t)n * n;
+  const cf one = mk(1.f), zero = mk(0.f);
+  MX_EW(k_to_double, bm * nn, bm * nn, r.W32, W64);
+  MX_EW(k_to_double, bm * n, bm * n, r.lam32, r.mu);
+  // the FP32 products (E = W^-1 R, W F): 3xTF32 on the tensor cores when the recursion's products
+  // are (their planes are free until the recursion), else the tiled product
+  auto mode_prod = [&](const cf* A, const cf* B, cf* C) -> int {
+    if (!r.tfA) return launch_gemm<float>(bm, n, n, n, one, A, n, nn, B, n, nn, zero, C, n, nn, s);
+    int st = tf32x3_split_a(bm, n, n, A, n, nn, nullptr, r.tfA, s);
+    if (!st) st = tf32x3_split_b(bm, n, n, B, n, nn, nullptr, zero, r.tfB, s);
+    return st ? st : tf32x3_from_planes(bm, n, n, n, r.tfA, r.tfB, one, zero, C, n, nn, r.tferr, s);
+  };
+  // M W in FP64 (tensor-core digit products) at every step.  Updating it in FP32 instead
+  // (M W += round(M W) F) is only FP32-accurate where F is large: next to a nearly defective
+  // cluster that error enters the next step's residual and the refinement stalls at ~1e-8.
+  // (The structured product P (Q W) costs less but cancels terms of size k^4 / eps for the
+  // evanescent orders.)
+  for (int step = 0; step < kEigSteps; ++step) {
+    // E with the inverse of the current W: the first step can rotate the vectors of a close
+    // pair by ~1e-3, after which W0^-1 would make the later steps converge only linearly
+    MX_TRY(launch_copy<float>(bm, n, n, r.W32, n, nn, r.lu32, n, nn, s));
+    MX_TRY(launch_inverse_blocked<float>(bm, n, r.lu32, n, nn, r.Wi, n, nn, r.piv, r.st, s));
+    MX_TRY(ozaki_zgemm(bm, n, n, n, M64, n, nn, nullptr, W64, n, nn, r.MW64, n, nn, r.oz, s, mode_step_digits()));
+    MX_PP(k_eig_residual, bm, nn, n, r.MW64, W64, r.mu, r.E32);
+    MX_TRY(mode_prod(r.Wi, r.E32, r.Z32));  // E
+    MX_TRY(launch_clusters(bm, n, r.mu, r.Z32, r.pair, r.nearest, r.csz, r.memb, r.xc, r.mu_next, s));
+    MX_PP(k_eig_update, bm, nn, n, r.mu, r.Z32, r.F32, r.pair, r.nearest, r.csz, r.memb, r.xc);
+    MX_TRY(mode_prod(r.W32, r.F32, r.Z32));
+    MX_EW(k_add_correction, bm * nn, bm * nn, W64, r.Z32, r.W32);
+    std::swap(r.mu, r.mu_next);
+  }
+  return KHP_OK;
+}
+
+// Workspace of launch_geev_refined.
+struct RefinedWs {
+  EigRefine er;
+  cf* M32;   // with Z32 one block: Z of the FP64 eigensolver
+  cf* lam32;
+  int *st, *act;
+};
+
+RefinedWs plan_refined(Arena& a, int64_t batch, int n) {
+  const size_t nn = (size_t)n * n, b = (size_t)batch;
+  RefinedWs w;
+  EigRefine& r = w.er;
+  w.M32 = a.take<cf>(2 * b * nn);
+  r.F32 = w.M32;
+  r.Z32 = w.M32 ? w.M32 + b * nn : nullptr;
+  r.W32 = a.take<cf>(b * nn);
+  r.Wi = a.take<cf>(b * nn);
+  r.E32 = a.take<cf>(b * nn);
+  r.lu32 = a.take<cf>(b * nn);
+  r.MW64 = a.take<cd>(b * nn);
+  r.mu = a.take<cd>(b * n);
+  r.mu_next = a.take<cd>(b * n);
+  w.lam32 = a.take<cf>(b * n);
+  r.lam32 = w.lam32;
+  r.pair = a.take<int>(b * n);
+  r.nearest = a.take<int>(b * n);
+  r.csz = a.take<int>(b * n);
+  r.memb = a.take<int>(b * n * kClusterMax);
+  r.xc = a.take<cf>(b * n * kClusterMax);
+  r.piv = a.take<int>(b * n);
+  w.st = a.take<int>(b);
+  w.act = a.take<int>(b);
+  r.st = w.st;
+  const size_t ch = (size_t)ozaki_chunk((int64_t)b);
+  r.oz.ad_elems = ch * ozaki_a_elems(n, n);
+  r.oz.ad = a.take<uint16_t>(r.oz.ad_elems);
+  r.oz.ea_n = ch * ozaki_rows_padded(n);
+  r.oz.ea = a.take<int>(r.oz.ea_n);
+  r.oz.bd_elems = ch * ozaki_b_elems(n, n);
+  r.oz.bd = a.take<uint16_t>(r.oz.bd_elems);
+  r.oz.eb_n = ch * n;
+  r.oz.eb = a.take<int>(r.oz.eb_n);
+  r.oz.err = a.take<int>(1);
+  r.tfA = r.tfB = nullptr;
+  r.tferr = nullptr;
+  if (use_tf32_products(n)) {
+    r.tfA = a.take<float>(b * tf32x3_a_elems(n, n));
+    r.tfB = a.take<float>(b * tf32x3_b_elems(n, n));
+    r.tferr = a.take<int>(1);
+  }
+  return w;
+}
+
 // Backward stage of khp_solve_batched_mixed_grad (after the forward refinement): loss seeds,
 // the adjoint solve (FP64 transposed residual + FP32 transposed sweep, refine + 3 rounds), the
 // per-layer M-gradients and the convolution-matrix gradient of every map.
@@ -1482,50 +1611,14 @@ int solve_mixed(int64_t batch, int px, int py, int L, const int* kinds, const in
     MX_TRY(launch_geev<float>(bm, n, p.M32, n, nn, p.Z32, W32, n, nn, lam32, n, sx, s, p.M64,
                               (int64_t)(2 * nn * sizeof(cd))));
     stage_end(KHP_STAGE_EIGENSOLVE, s);
-    // Refinement steps: R = M W - W mu in FP64, E = W^-1 R (FP32 inverse of the current W, held
-    // in Wi until the final inverse), mu += diag(E), W += W F.
     MX_TRY(launch_assemble_pq<double>(bm, nh, Cm, HX, HY, midx, gx, gy, kpx, k0x, p.M64, s));
-    MX_EW(k_to_double, bm * nn, bm * nn, W32, W64);
-    MX_EW(k_to_double, bm * n, bm * n, lam32, p.mu64);
-    MX_TRY(launch_copy<float>(bm, n, n, W32, n, nn, p.lu32, n, nn, s));
-    MX_TRY(launch_inverse_blocked<float>(bm, n, p.lu32, n, nn, Wi, n, nn, p.piv, sx, s));
-    cd* mu_a = p.mu64;
-    cd* mu_b = p.mu64b;
-    // the refinement steps' FP32 products (E = W^-1 R, W F): 3xTF32 on the tensor cores when the
-    // recursion's products are (their planes are free until the recursion), else the tiled product
-    auto mode_prod = [&](const cf* A, const cf* B, cf* C) -> int {
-      if (!p.tfA) return launch_gemm<float>(bm, n, n, n, one, A, n, nn, B, n, nn, zero, C, n, nn, s);
-      int st = tf32x3_split_a(bm, n, n, A, n, nn, nullptr, p.tfA, s);
-      if (!st) st = tf32x3_split_b(bm, n, n, B, n, nn, nullptr, zero, p.tfB, s);
-      return st ? st : tf32x3_from_planes(bm, n, n, n, p.tfA, p.tfB, one, zero, C, n, nn, p.tferr, s);
-    };
-    // M W in FP64 (tensor-core digit products) at every step.  Updating it in FP32 instead
-    // (M W += round(M W) F) is only FP32-accurate where F is large: next to a nearly defective
-    // cluster that error enters the next step's residual and the refinement stalls at ~1e-8.
-    // (The structured product P (Q W) costs less but cancels terms of size k^4 / eps for the
-    // evanescent orders.)
-    for (int step = 0; step < kEigSteps; ++step) {
-      if (step > 0) {
-        // E with the inverse of the current W: the first step can rotate the vectors of a close
-        // pair by ~1e-3, after which W0^-1 would make the later steps converge only linearly
-        MX_TRY(launch_copy<float>(bm, n, n, W32, n, nn, p.lu32, n, nn, s));
-        MX_TRY(launch_inverse_blocked<float>(bm, n, p.lu32, n, nn, Wi, n, nn, p.piv, sx, s));
-      }
-      MX_TRY(ozaki_zgemm(bm, n, n, n, p.M64, n, nn, nullptr, W64, n, nn, p.MW64, n, nn, p.oz, s,
-                         mode_step_digits()));
-      MX_PP(k_eig_residual, bm, nn, n, p.MW64, W64, mu_a, p.E32);
-      MX_TRY(mode_prod(Wi, p.E32, p.Z32));  // E
-      MX_TRY(launch_clusters(bm, n, mu_a, p.Z32, p.pair, p.nearest, p.csz, p.memb, p.xc, mu_b, s));
-      MX_PP(k_eig_update, bm, nn, n, mu_a, p.Z32, p.M32, p.pair, p.nearest, p.csz, p.memb, p.xc);  // M32 <- F
-      MX_TRY(mode_prod(W32, p.M32, p.Z32));
-      MX_EW(k_add_correction, bm * nn, bm * nn, W64, p.Z32, W32);
-      std::swap(mu_a, mu_b);
-    }
+    EigRefine er{W32,  Wi,     p.Z32, p.E32,  p.lu32, p.M32, lam32, p.MW64, p.mu64, p.mu64b, p.pair, p.nearest,
+                 p.csz, p.memb, p.xc,  p.piv, sx,     p.tfA, p.tfB, p.tferr, p.oz};
+    MX_TRY(refine_eigs(bm, n, p.M64, W64, er, s));
+    const cd* mu_a = er.mu;
     // FP64 eigen-residual of the refined modes (KHP_BIT_MODES where a column missed 1e-8)
     MX_TRY(ozaki_zgemm(bm, n, n, n, p.M64, n, nn, nullptr, W64, n, nn, p.MW64, n, nn, p.oz, s));
-    k_eig_check<<<(unsigned)bm, 256, 0, s>>>(n, p.MW64, W64, mu_a, kpx, k0x, epsi, sx);
-    count_launches(1);
-    MX_TRY(cuda_status());
+    MX_TRY(launch_eig_check(bm, n, p.MW64, W64, mu_a, kpx, k0x, epsi, 1e-8, KHP_BIT_MODES, sx, s));
     MX_EW(k_sqrt_mu, bm * n, bm * n, mu_a, lam64, lam32);
     // V = Q W / lam in FP64
     cd* CWt = p.CW64;
@@ -1693,6 +1786,59 @@ int solve_mixed(int64_t batch, int px, int py, int L, const int* kinds, const in
 }
 
 }  // namespace
+
+// FP64 eigenpairs: the FP32 eigensolver refined in FP64, with the FP64 eigensolver for the matrices
+// whose refined residual is above what the FP64 QR itself leaves (measured over symmetric, multi-disc and
+// lossy maps: max|M W - W mu| / (max|mu| max|W|) up to 5e-15 at n = 18, 2e-14 at n = 98 and 1e-13 at
+// n = 242; refined: the same or less).  The FP64 QR is one CTA's chain on a pipe of 2 FMAs per clock:
+// one matrix takes 15 to 21 ms at n = 50, 60 to 77 at n = 98 and 410 to 510 at n = 242, against 3.1, 8
+// to 9 and 43 to 47 here; 64 matrices of n = 126 112 against 15 ms.  A nearly uniform symmetric map,
+// whose exactly degenerate groups are larger than a cluster, pays for both (9.4 against 12.4 ms at
+// n = 50).  Below kRefinedMinN the FP64 QR alone is as fast (n = 10: 0.7 ms each way, n = 18: 2.3
+// against 1.0).
+constexpr int kRefinedMinN = 12;
+constexpr int kRefinedMaxN = 4096;  // the digit products' limit
+constexpr double kRefinedTolPerN = 2e-16;
+
+size_t geev_refined_workspace(int64_t batch, int n) {
+  Arena a{nullptr, 0};
+  if (n < kRefinedMinN || n > kRefinedMaxN) {
+    a.take<cd>((size_t)batch * n * n);  // Z
+  } else {
+    plan_refined(a, batch, n);
+  }
+  return a.off;
+}
+
+int launch_geev_refined(int64_t batch, int n, cd* M, cd* W, cd* lam, int* info, cudaStream_t s, void* ws,
+                        size_t ws_bytes) {
+  if (batch <= 0) return KHP_OK;
+  const int64_t nn = (int64_t)n * n;
+  Arena a{static_cast<char*>(ws), ws_bytes};
+  if (n < kRefinedMinN || n > kRefinedMaxN) {
+    cd* Z = a.take<cd>((size_t)batch * nn);
+    if (!a.ok || !ws) return KHP_ERR_WORKSPACE;
+    return launch_geev<double>(batch, n, M, n, nn, Z, W, n, nn, lam, n, info, s);
+  }
+  RefinedWs w = plan_refined(a, batch, n);
+  if (!a.ok || !ws) return KHP_ERR_WORKSPACE;
+  EigRefine& r = w.er;
+  if (cudaMemsetAsync(w.st, 0, sizeof(int) * batch, s) != cudaSuccess) return KHP_ERR_CUDA;
+  MX_EW(k_round, batch * nn, batch * nn, M, w.M32);
+  MX_TRY(launch_geev<float>(batch, n, w.M32, n, nn, r.Z32, r.W32, n, nn, w.lam32, n, w.st, s, r.MW64,
+                            (int64_t)(nn * sizeof(cd)) / 32 * 32));
+  MX_TRY(refine_eigs(batch, n, M, W, r, s));
+  MX_TRY(ozaki_zgemm(batch, n, n, n, M, n, nn, nullptr, W, n, nn, r.MW64, n, nn, r.oz, s));
+  // matrices to solve in FP64 after all: an FP32 stage failed, or a column's residual is too large
+  if (cudaMemcpyAsync(w.act, w.st, sizeof(int) * batch, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+    return KHP_ERR_CUDA;
+  MX_TRY(launch_eig_check(batch, n, r.MW64, W, r.mu, nullptr, nullptr, mk(0.0), kRefinedTolPerN * n, 1, w.act, s));
+  if (cudaMemcpyAsync(lam, r.mu, sizeof(cd) * batch * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+    return KHP_ERR_CUDA;
+  MX_TRY(launch_normalize_cols<double>(batch, n, W, n, nn, s));
+  return launch_geev<double>(batch, n, M, n, nn, reinterpret_cast<cd*>(w.M32), W, n, nn, lam, n, info, s, nullptr, 0,
+                             w.act);
+}
 
 int mixed_modes_in_workspace(int64_t batch, int nh, int L, const int* kinds, const int* maps, const void* ws,
                              size_t ws_bytes, const cd** W, const cd** V, const cd** lam) {

@@ -583,7 +583,8 @@ inline PrepWs plan_prep(Arena& a, int64_t nmaps, int nh) {
 
 struct ModesWs {
   cd* M;
-  cd* Z;
+  char* eig;
+  size_t eig_bytes;
   cd* CWt;
   cd* CWb;
 };
@@ -591,7 +592,8 @@ inline ModesWs plan_modes(Arena& a, int64_t batch, int nh) {
   const size_t n = 2 * (size_t)nh;
   ModesWs w;
   w.M = a.take<cd>(batch * n * n);
-  w.Z = a.take<cd>(batch * n * n);
+  w.eig_bytes = geev_refined_workspace(batch, (int)n);
+  w.eig = a.take<char>(w.eig_bytes);
   w.CWt = a.take<cd>(batch * nh * n);
   w.CWb = a.take<cd>(batch * nh * n);
   return w;
@@ -805,7 +807,7 @@ int khp_layer_modes(int64_t batch, int32_t nh, const int32_t* map_index, const d
                                                      (const cd*)hy, gx, gy, kp, k0, w.M);
   count_launches(1);
   KHP_TRY(cuda_status());
-  KHP_TRY(launch_geev<double>(batch, n, w.M, n, nn, w.Z, (cd*)W, n, nn, (cd*)lam, n, status, s));
+  KHP_TRY(launch_geev_refined(batch, n, w.M, (cd*)W, (cd*)lam, status, s, w.eig, w.eig_bytes));
   k_sqrt_lam<<<ew_grid(batch * n), 256, 0, s>>>(batch * n, (cd*)lam);
   count_launches(1);
   KHP_TRY(launch_gemm<double>(batch, nh, n, nh, mk(1.0), (const cd*)conv, nh, hh, (const cd*)W, n, nn, mk(0.0), w.CWt,
