@@ -4,6 +4,7 @@
 
 #include "khepri_gb300.h"
 #include "khp_dense.cuh"
+#include "khp_hqr.cuh"
 #include "khp_launch.h"
 
 namespace khp {
@@ -18,6 +19,7 @@ constexpr int64_t kMaxGridY = 65535;
 constexpr int kTuneMaxN = 4096;
 int g_eig_threads[kTuneMaxN + 1] = {0};
 
+bool eig_tuned(int n) { return n <= kTuneMaxN && g_eig_threads[n] > 0; }
 int eig_threads(int n) {
   const int v = n <= kTuneMaxN ? g_eig_threads[n] : 0;
   return v > 0 ? v : kTeamThreads;
@@ -72,18 +74,29 @@ __global__ void __launch_bounds__(kTeamThreads, 3) k_gehrd(int n, cplx<T>* A, in
     team_gehrd(t, A + b * bsA, lda, n, Z + b * (int64_t)n * n, n, reinterpret_cast<cplx<T>*>(dyn), &sh);
 }
 
+// Window scratch of team_hqr_win.
+template <typename T>
+struct HqrWindow {
+  cplx<T> win[(KHP_HQR_WIN + 2) * (KHP_HQR_WIN + 2)], rs[KHP_HQR_WIN];
+  T rc[KHP_HQR_WIN];
+};
+template <typename T>
+size_t schur_smem(int n, bool log) {
+  if constexpr (sizeof(T) == 4)
+    if (log) return sizeof(HqrShared<T>) + hqr_strip_smem<T>(n);
+  return sizeof(HqrWindow<T>);
+}
+
 // Schur form of the Hessenberg matrix and eigenvectors of the triangular factor (X left in A,
 // Q in Z); the back-transform W = Z X runs afterwards as a batched tiled product.  With a log
 // region (log_bytes per matrix at logbuf) Z's updates are logged and left for k_hqr_apply_log.
 template <typename T>
-__global__ void __launch_bounds__(kTeamThreads) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
+__global__ void __launch_bounds__(kTeamThreads + 32, sizeof(T) == 4 ? 2 : 1) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
                                                               cplx<T>* lam, int64_t bsLam, int* info,
                                                               unsigned char* logbuf, int64_t log_bytes,
                                                               const int* __restrict__ only) {
-  __shared__ TeamShared sh;
-  __shared__ cplx<T> win[(KHP_HQR_WIN + 2) * (KHP_HQR_WIN + 2)];
-  __shared__ cplx<T> rs[KHP_HQR_WIN];
-  __shared__ T rc[KHP_HQR_WIN];
+  __shared__ TeamShared ts;
+  extern __shared__ __align__(16) unsigned char dyn[];  // schur_smem<T>
   TeamCta t;
   const int64_t b = blockIdx.x;
   if (only && !only[b]) return;
@@ -92,9 +105,16 @@ __global__ void __launch_bounds__(kTeamThreads) k_geev_schur(int n, cplx<T>* A, 
   int st;
   if (logbuf) {
     const HqrLog<T> L = hqr_log_view<T>(logbuf + b * log_bytes, log_bytes, n);
-    st = team_hqr_win(t, Ab, lda, n, Zb, n, win, rc, rs, &sh, &L);
+    if constexpr (sizeof(T) == 4) {
+      HqrShared<T>& hs = *reinterpret_cast<HqrShared<T>*>(dyn);
+      st = cta_hqr(Ab, lda, n, Zb, n, hs, reinterpret_cast<cplx<T>*>(dyn + sizeof(HqrShared<T>)), L);
+    } else {
+      HqrWindow<T>& hw = *reinterpret_cast<HqrWindow<T>*>(dyn);
+      st = team_hqr_win(t, Ab, lda, n, Zb, n, hw.win, hw.rc, hw.rs, &ts, &L);
+    }
   } else {
-    st = team_hqr_win(t, Ab, lda, n, Zb, n, win, rc, rs, &sh);
+    HqrWindow<T>& hw = *reinterpret_cast<HqrWindow<T>*>(dyn);
+    st = team_hqr_win(t, Ab, lda, n, Zb, n, hw.win, hw.rc, hw.rs, &ts);
   }
   team_trevc(t, Ab, lda, n, lam + b * bsLam);
   if (threadIdx.x == 0 && st) info[b] |= st;
@@ -851,7 +871,20 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   if (logbuf && !only && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
       hqr_log_view<T>(logbuf, log_bytes, n).cap_rot >= n - 1)
     lg = static_cast<unsigned char*>(logbuf);
-  k_geev_schur<T><<<(unsigned)batch, threads, 0, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes,
+  const size_t ssm = schur_smem<T>(n, lg != nullptr);
+  if (ssm > 40 * 1024 &&
+      cudaFuncSetAttribute(k_geev_schur<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm) != cudaSuccess)
+    return KHP_ERR_CUDA;
+  // FP32: a warp for the chase and, up to 288 threads, one per strip; fewer strips than threads still
+  // gain (eigenvectors of the triangular factor): n = 50, 151 matrices: 128 threads 781 us, 256 626;
+  // n = 98, 64: 160 threads 2.40 ms, 256 1.88; n = 242, 912: 256 threads 53.8 ms, 288 51.8; n = 18, 512:
+  // 128 threads 325 us, 256 425
+  const int sthreads = sizeof(T) == 8 || !lg ? threads
+                       : eig_tuned(n)        ? std::max(64, threads)
+                       : n <= 32             ? 128
+                       : n <= 224            ? kTeamThreads
+                                             : kTeamThreads + 32;
+  k_geev_schur<T><<<(unsigned)batch, sthreads, ssm, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes,
                                                        only);
   count_launches(2);
   int st = cuda_status();
