@@ -1372,9 +1372,9 @@ int launch_eig_check(int64_t batch, int n, const cd* MW, const cd* W, const cd* 
 }
 
 // Eigenpairs of the FP64 matrices M from an FP32 eigensolver's (r.W32, r.lam32): W64 and r.mu, by
-// kEigSteps steps of R = M W - W mu in FP64, E = W^-1 R (FP32 inverse of the current W, left in r.Wi),
+// `steps` steps of R = M W - W mu in FP64, E = W^-1 R (FP32 inverse of the current W, left in r.Wi),
 // mu += diag(E), W += W F.
-int refine_eigs(int64_t bm, int n, const cd* M64, cd* W64, EigRefine& r, cudaStream_t s) {
+int refine_eigs(int64_t bm, int n, const cd* M64, cd* W64, EigRefine& r, int steps, cudaStream_t s) {
   const int64_t nn = (int64_t)n * n;
   const cf one = mk(1.f), zero = mk(0.f);
   MX_EW(k_to_double, bm * nn, bm * nn, r.W32, W64);
@@ -1392,7 +1392,7 @@ int refine_eigs(int64_t bm, int n, const cd* M64, cd* W64, EigRefine& r, cudaStr
   // cluster that error enters the next step's residual and the refinement stalls at ~1e-8.
   // (The structured product P (Q W) costs less but cancels terms of size k^4 / eps for the
   // evanescent orders.)
-  for (int step = 0; step < kEigSteps; ++step) {
+  for (int step = 0; step < steps; ++step) {
     // E with the inverse of the current W: the first step can rotate the vectors of a close
     // pair by ~1e-3, after which W0^-1 would make the later steps converge only linearly
     MX_TRY(launch_copy<float>(bm, n, n, r.W32, n, nn, r.lu32, n, nn, s));
@@ -1614,7 +1614,7 @@ int solve_mixed(int64_t batch, int px, int py, int L, const int* kinds, const in
     MX_TRY(launch_assemble_pq<double>(bm, nh, Cm, HX, HY, midx, gx, gy, kpx, k0x, p.M64, s));
     EigRefine er{W32,  Wi,     p.Z32, p.E32,  p.lu32, p.M32, lam32, p.MW64, p.mu64, p.mu64b, p.pair, p.nearest,
                  p.csz, p.memb, p.xc,  p.piv, sx,     p.tfA, p.tfB, p.tferr, p.oz};
-    MX_TRY(refine_eigs(bm, n, p.M64, W64, er, s));
+    MX_TRY(refine_eigs(bm, n, p.M64, W64, er, kEigSteps, s));
     const cd* mu_a = er.mu;
     // FP64 eigen-residual of the refined modes (KHP_BIT_MODES where a column missed 1e-8)
     MX_TRY(ozaki_zgemm(bm, n, n, n, p.M64, n, nn, nullptr, W64, n, nn, p.MW64, n, nn, p.oz, s));
@@ -1798,7 +1798,8 @@ int solve_mixed(int64_t batch, int px, int py, int L, const int* kinds, const in
 // against 1.0).
 constexpr int kRefinedMinN = 12;
 constexpr int kRefinedMaxN = 4096;  // the digit products' limit
-constexpr double kRefinedTolPerN = 2e-16;
+constexpr double kRefinedTolPerN = 4e-16;
+constexpr int kRefinedSteps = 4;
 
 size_t geev_refined_workspace(int64_t batch, int n) {
   Arena a{nullptr, 0};
@@ -1827,7 +1828,7 @@ int launch_geev_refined(int64_t batch, int n, cd* M, cd* W, cd* lam, int* info, 
   MX_EW(k_round, batch * nn, batch * nn, M, w.M32);
   MX_TRY(launch_geev<float>(batch, n, w.M32, n, nn, r.Z32, r.W32, n, nn, w.lam32, n, w.st, s, r.MW64,
                             (int64_t)(nn * sizeof(cd)) / 32 * 32));
-  MX_TRY(refine_eigs(batch, n, M, W, r, s));
+  MX_TRY(refine_eigs(batch, n, M, W, r, kRefinedSteps, s));
   MX_TRY(ozaki_zgemm(batch, n, n, n, M, n, nn, nullptr, W, n, nn, r.MW64, n, nn, r.oz, s));
   // matrices to solve in FP64 after all: an FP32 stage failed, or a column's residual is too large
   if (cudaMemcpyAsync(w.act, w.st, sizeof(int) * batch, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
