@@ -297,6 +297,8 @@ __global__ void __launch_bounds__(256) k_gemm(int n, int m, int k, cplx<T> alpha
     stage();
     __syncthreads();
     if (kPrefetch && k0 + BK < k) load(k0 + BK);
+    // (FP64: a warp whose two rows lie past the matrix leaves the pipe to the others)
+    if (sizeof(T) == 4 || row0 + (ty & ~1) < n)
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       cplx<T> a[TM], bb[TN];
@@ -825,24 +827,31 @@ int launch_gemm(int64_t batch, int n, int m, int k, cplx<T> alpha, const cplx<T>
                 const cplx<T>* B, int64_t ldb, int64_t bsB, cplx<T> beta, cplx<T>* C, int64_t ldc, int64_t bsC,
                 cudaStream_t s, const int* aidx, const int* bidx, cplx<T> bshift, const int* only) {
   if (batch <= 0 || n <= 0 || m <= 0) return KHP_OK;
-  // 64 x 64 tiles (4 x 4 outputs per thread) once both output dimensions reach 64; 32 x 128
+  // FP64: 16 x 16 tiles.  The FP64 pipe (2 FMAs per clock and SM) bounds these whatever the tile, so the
+  // smallest tile wastes least on padding and spreads one product over the most SMs (one 50 x 50 product
+  // 66 us on the 4 SMs of 32 x 32 tiles, 19 here; 64 products of n = 98 0.80 ms at 64 x 64 tiles, 0.40).
+  // FP32: 64 x 64 tiles (4 x 4 outputs per thread) once both output dimensions reach 64; 32 x 128
   // (2 x 8) for outputs of at most 32 rows and at least 128 columns (the block rows of the
   // substitutions); else 32 x 32
-  const bool big = n >= 64 && m >= 64;
-  const bool wide = !big && n <= 32 && m >= 128;
-  const int BM = big ? 64 : 32, BN = big ? 64 : wide ? 128 : 32;
+  const bool big = sizeof(T) == 4 && n >= 64 && m >= 64;
+  const bool wide = sizeof(T) == 4 && !big && n <= 32 && m >= 128;
+  const int BM = sizeof(T) == 8 ? 16 : big ? 64 : 32, BN = sizeof(T) == 8 ? 16 : big ? 64 : wide ? 128 : 32;
   for (int64_t off = 0; off < batch; off += kMaxGridY) {
     const unsigned nb = (unsigned)std::min<int64_t>(batch - off, kMaxGridY);
     dim3 grid((m + BN - 1) / BN, (n + BM - 1) / BM, nb);
-    if (wide)
+    if constexpr (sizeof(T) == 8) {
+      k_gemm<T, 16, 16, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
+                                                 aidx, bidx, bshift, only);
+    } else if (wide) {
       k_gemm<T, 32, 128, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
                                                   aidx, bidx, bshift, only);
-    else if (big)
+    } else if (big) {
       k_gemm<T, 64, 64, 8><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
                                                 aidx, bidx, bshift, only);
-    else
+    } else {
       k_gemm<T, 32, 32, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
                                                  aidx, bidx, bshift, only);
+    }
     count_launches(1);
   }
   return cuda_status();

@@ -14,7 +14,7 @@
 //       Gamma <- (P1 + P2)(P1 - P2)^-1;
 //   forward, from the incidence side, the right-going amplitudes of the two source columns:
 //       homogeneous: u <- M^-1 S21 u;  patterned: u <- 2 (F - G)^-1 X 2 (P1 - P2)^-1 u,
-//   with the LU factors kept from the backward pass; finally r = S11 c + S12 Gamma u at the
+//   with the inverses kept from the backward pass; finally r = S11 c + S12 Gamma u at the
 //   incidence half-space and t = S21 u at the emergence half-space.
 //
 // Exactly equivalent to the reference's chain (same continuity conditions), ~2.8x fewer flops
@@ -61,13 +61,11 @@ struct GammaPlan {
   size_t eig_bytes;
   std::vector<int*> midx;  // per distinct map: the map index of every problem
   // per layer
-  std::vector<cplx<T>*> lu1, lu2;
-  std::vector<int*> piv1, piv2;
+  std::vector<cplx<T>*> inv1, inv2;  // explicit inverses of the recursion's matrices
   std::vector<M2*> blocks;  // homogeneous layers
   M2 *inc, *trn;
   cplx<T> *G, *F, *Gb, *P;
   cplx<T> *u, *tmp, *rv, *tv;
-  int* pivs;
   M2 *v0b, *v0ib;  // free-space blocks per problem and harmonic
 };
 
@@ -93,16 +91,12 @@ GammaPlan<T> plan_gamma(Arena& a, int64_t batch, int nh, int nlayers, const int*
   p.piv = a.take<int>(batch * n);
   for (int l = 0; l < nlayers; ++l) {
     if (kinds[l] == 1) {
-      p.lu1.push_back(a.take<cplx<T>>(batch * nn));
-      p.lu2.push_back(a.take<cplx<T>>(batch * nn));
-      p.piv1.push_back(a.take<int>(batch * n));
-      p.piv2.push_back(a.take<int>(batch * n));
+      p.inv1.push_back(a.take<cplx<T>>(batch * nn));
+      p.inv2.push_back(a.take<cplx<T>>(batch * nn));
       p.blocks.push_back(nullptr);
     } else {
-      p.lu1.push_back(a.take<cplx<T>>(batch * nn));
-      p.lu2.push_back(nullptr);
-      p.piv1.push_back(a.take<int>(batch * n));
-      p.piv2.push_back(nullptr);
+      p.inv1.push_back(a.take<cplx<T>>(batch * nn));
+      p.inv2.push_back(nullptr);
       p.blocks.push_back(a.take<M2>(batch * nh * 4));
     }
   }
@@ -116,18 +110,9 @@ GammaPlan<T> plan_gamma(Arena& a, int64_t batch, int nh, int nlayers, const int*
   p.tmp = a.take<cplx<T>>(batch * n * 2);
   p.rv = a.take<cplx<T>>(batch * n * 2);
   p.tv = a.take<cplx<T>>(batch * n * 2);
-  p.pivs = a.take<int>(batch * n);
   p.v0b = a.take<M2>(batch * nh);
   p.v0ib = a.take<M2>(batch * nh);
   return p;
-}
-
-template <typename T>
-int launch_getrs_right(int64_t batch, int n, const cplx<T>* A, int64_t lda, int64_t bsA, const int* piv, cplx<T>* B,
-                       int64_t ldb, int64_t bsB, int m, cudaStream_t s) {
-  k_getrs_right<T><<<(unsigned)batch, 256, 0, s>>>(n, A, lda, bsA, piv, B, ldb, bsB, m);
-  count_launches(1);
-  return cuda_status();
 }
 
 #define GT_TRY(x)        \
@@ -221,9 +206,9 @@ int solve_gamma(int64_t batch, int px, int py, int nlayers, const int* kinds, co
       GT_TRY(launch_modes_v<T>(batch, nh, gx, gy, kp, k0, p.W[m], CWt, CWb, hn, p.lam[m], p.V[m], status, s));
     }
     GT_TRY(launch_copy<T>(batch, n, n, p.W[m], n, nn, p.lu, n, nn, s));
-    GT_TRY(launch_inverse<T>(batch, n, p.lu, n, nn, p.Wi[m], n, nn, p.piv, status, s));
+    GT_TRY(launch_inverse_blocked<T>(batch, n, p.lu, n, nn, p.Wi[m], n, nn, p.piv, status, s));
     GT_TRY(launch_copy<T>(batch, n, n, p.V[m], n, nn, p.lu, n, nn, s));
-    GT_TRY(launch_inverse<T>(batch, n, p.lu, n, nn, p.Z, n, nn, p.piv, status, s));  // Z = V^-1
+    GT_TRY(launch_inverse_blocked<T>(batch, n, p.lu, n, nn, p.Z, n, nn, p.piv, status, s));  // Z = V^-1
     GT_EW(k_v0_right<T>, batch * nn, batch, nh, p.v0b, p.Z, p.Q0[m]);
     GT_EW(k_v0inv_left<T>, batch * nn, batch, nh, p.v0ib, p.V[m], p.Vt[m]);
   }
@@ -238,10 +223,10 @@ int solve_gamma(int64_t batch, int px, int py, int nlayers, const int* kinds, co
   GT_EW(k_gamma_from_blocks<T>, batch * nn, batch, nh, p.trn, 0, p.G);
   for (int l = nlayers - 1; l >= 0; --l) {
     if (kinds[l] != 1) {
-      GT_TRY(launch_i_minus_sg<T>(batch, nh, p.blocks[l], p.G, p.lu1[l], s));
-      GT_TRY(launch_getrf<T>(batch, n, p.lu1[l], n, nn, p.piv1[l], status, s));
-      GT_TRY(launch_getrs_right<T>(batch, n, p.lu1[l], n, nn, p.piv1[l], p.G, n, nn, n, s));  // G <- G M^-1
-      GT_TRY(launch_sandwich<T>(batch, nh, p.blocks[l], p.G, p.F, s));
+      GT_TRY(launch_i_minus_sg<T>(batch, nh, p.blocks[l], p.G, p.lu, s));
+      GT_TRY(launch_inverse_blocked<T>(batch, n, p.lu, n, nn, p.inv1[l], n, nn, p.piv, status, s));
+      GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.G, n, nn, p.inv1[l], n, nn, zero, p.P, n, nn, s));  // G M^-1
+      GT_TRY(launch_sandwich<T>(batch, nh, p.blocks[l], p.P, p.F, s));
       std::swap(p.G, p.F);
     } else {
       const int m = slot[l];
@@ -250,39 +235,40 @@ int solve_gamma(int64_t batch, int px, int py, int nlayers, const int* kinds, co
       GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.Wi[m], n, nn, p.G, n, nn, one, p.F, n, nn, s));
       GT_TRY(launch_copy<T>(batch, n, n, p.Q0[m], n, nn, p.Gb, n, nn, s));
       GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.Q0[m], n, nn, p.G, n, nn, mone, p.Gb, n, nn, s));
-      GT_EW(k_diff_sum<T>, batch * nn, batch * nn, p.F, p.Gb, p.lu1[l]);  // lu1 = F - G, F <- F + G
-      GT_TRY(launch_getrf<T>(batch, n, p.lu1[l], n, nn, p.piv1[l], status, s));
-      GT_TRY(launch_getrs_right<T>(batch, n, p.lu1[l], n, nn, p.piv1[l], p.F, n, nn, n, s));  // rho
+      GT_EW(k_diff_sum<T>, batch * nn, batch * nn, p.F, p.Gb, p.lu);  // lu = F - G, F <- F + G
+      GT_TRY(launch_inverse_blocked<T>(batch, n, p.lu, n, nn, p.inv1[l], n, nn, p.piv, status, s));
+      GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.F, n, nn, p.inv1[l], n, nn, zero, p.M, n, nn, s));  // rho
       GT_EW(k_xvec<T>, batch * n, batch, n, p.lam[m], depth_of(l), k0, p.u);                      // scratch
-      GT_EW(k_xmx_t<T>, batch * nn, batch, n, p.u, p.F);                                           // rho_L
+      GT_EW(k_xmx_t<T>, batch * nn, batch, n, p.u, p.M);                                           // rho_L
       GT_TRY(launch_copy<T>(batch, n, n, p.W[m], n, nn, p.Gb, n, nn, s));
-      GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.W[m], n, nn, p.F, n, nn, one, p.Gb, n, nn, s));    // P1
+      GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.W[m], n, nn, p.M, n, nn, one, p.Gb, n, nn, s));    // P1
       GT_TRY(launch_copy<T>(batch, n, n, p.Vt[m], n, nn, p.P, n, nn, s));
-      GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.Vt[m], n, nn, p.F, n, nn, mone, p.P, n, nn, s));   // P2
-      GT_EW(k_diff_sum<T>, batch * nn, batch * nn, p.Gb, p.P, p.lu2[l]);  // lu2 = P1 - P2, Gb <- P1 + P2
-      GT_TRY(launch_getrf<T>(batch, n, p.lu2[l], n, nn, p.piv2[l], status, s));
-      GT_TRY(launch_getrs_right<T>(batch, n, p.lu2[l], n, nn, p.piv2[l], p.Gb, n, nn, n, s));  // new Gamma
-      std::swap(p.G, p.Gb);
+      GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.Vt[m], n, nn, p.M, n, nn, mone, p.P, n, nn, s));   // P2
+      GT_EW(k_diff_sum<T>, batch * nn, batch * nn, p.Gb, p.P, p.lu);  // lu = P1 - P2, Gb <- P1 + P2
+      GT_TRY(launch_inverse_blocked<T>(batch, n, p.lu, n, nn, p.inv2[l], n, nn, p.piv, status, s));
+      GT_TRY(launch_gemm<T>(batch, n, n, n, one, p.Gb, n, nn, p.inv2[l], n, nn, zero, p.G, n, nn, s));  // new Gamma
     }
   }
   // ---- incidence half-space: M0 = I - S22 G, u = M0^-1 S21 c, r = S11 c + S12 G u ----
   GT_TRY(launch_i_minus_sg<T>(batch, nh, p.inc, p.G, p.lu, s));
-  GT_TRY(launch_getrf<T>(batch, n, p.lu, n, nn, p.pivs, status, s));
-  GT_EW(k_src_cols<T>, batch * n * 2, batch, nh, p.inc, 2, p.u);
-  GT_TRY(launch_getrs<T>(batch, n, p.lu, n, nn, p.pivs, p.u, 2, 2 * n, 2, s));
+  GT_TRY(launch_inverse_blocked<T>(batch, n, p.lu, n, nn, p.M, n, nn, p.piv, status, s));
+  GT_EW(k_src_cols<T>, batch * n * 2, batch, nh, p.inc, 2, p.tmp);
+  auto apply = [&](const cplx<T>* A, const cplx<T>* x, cplx<T>* y) {
+    return launch_gemm<T>(batch, n, 2, n, one, A, n, nn, x, 2, 2 * n, zero, y, 2, 2 * n, s);
+  };
+  GT_TRY(apply(p.M, p.tmp, p.u));
   GT_TRY(launch_gemm<T>(batch, n, 2, n, one, p.G, n, nn, p.u, 2, 2 * n, zero, p.tmp, 2, 2 * n, s));
   GT_EW(k_block_apply<T>, batch * n * 2, batch, nh, p.inc, 1, p.tmp, p.rv, 0);
   // ---- forward pass ----
   for (int l = 0; l < nlayers; ++l) {
     if (kinds[l] != 1) {
       GT_EW(k_block_apply<T>, batch * n * 2, batch, nh, p.blocks[l], 2, p.u, p.tmp, -1);
-      GT_TRY(launch_getrs<T>(batch, n, p.lu1[l], n, nn, p.piv1[l], p.tmp, 2, 2 * n, 2, s));
-      std::swap(p.u, p.tmp);
+      GT_TRY(apply(p.inv1[l], p.tmp, p.u));
     } else {
       const int m = slot[l];
-      GT_TRY(launch_getrs<T>(batch, n, p.lu2[l], n, nn, p.piv2[l], p.u, 2, 2 * n, 2, s));
-      GT_EW(k_vec_x4<T>, batch * n * 2, batch, n, p.lam[m], depth_of(l), k0, p.u);
-      GT_TRY(launch_getrs<T>(batch, n, p.lu1[l], n, nn, p.piv1[l], p.u, 2, 2 * n, 2, s));
+      GT_TRY(apply(p.inv2[l], p.u, p.tmp));
+      GT_EW(k_vec_x4<T>, batch * n * 2, batch, n, p.lam[m], depth_of(l), k0, p.tmp);
+      GT_TRY(apply(p.inv1[l], p.tmp, p.u));
     }
   }
   GT_EW(k_block_apply<T>, batch * n * 2, batch, nh, p.trn, 2, p.u, p.tv, -1);

@@ -49,14 +49,6 @@ __device__ __forceinline__ cd to_d(cplx<T> z) { return mk((double)z.re, (double)
 __device__ __forceinline__ cd blk(const M2& m, int r, int c) { return r == 0 ? (c == 0 ? m.a : m.b) : (c == 0 ? m.c : m.d); }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_getrs_right(int n, const cplx<T>* A, int64_t lda, int64_t bsA, const int* piv,
-                                                      cplx<T>* B, int64_t ldb, int64_t bsB, int m) {
-  TeamCta t;
-  const int64_t b = blockIdx.x;
-  team_getrs_right(t, A + b * bsA, lda, n, piv + b * n, B + b * bsB, ldb, m);
-}
-
-template <typename T>
 __global__ void k_convert(int64_t count, const cd* __restrict__ in, cplx<T>* out) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x)
     out[e] = to_t<T>(in[e]);

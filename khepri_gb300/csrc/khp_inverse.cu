@@ -344,21 +344,24 @@ __global__ void __launch_bounds__(MAXT) k_gj_panel(int n, int kb, int w, cplx<T>
 
 // The update of every row outside the panel [kb, kb + w), in place; or, for the last panel, from
 // A to out with the inverse's rows and columns interchanged (inv[p_r][k] = B[r][p_k]) and the pivot
-// columns read from A itself.  64 x 64 tiles, 4 x 4 outputs per thread, the whole rank in one pass
-// through shared memory.  Bound by reading and writing the matrix once per panel and by the issue of
+// columns read from A itself.  Tiles of 16 TM x 16 TN, TM x TN outputs per thread, the whole rank in one
+// pass through shared memory: 64 x 64 in FP32; 16 x 16 in FP64, whose pipe is so slow (2 FMAs per clock
+// and SM) that padding and idle SMs cost more than the extra loads.  Bound by reading and writing the matrix once per panel and by the issue of
 // the FMAs beside their shared-memory loads: 435 us for 912 matrices of n = 242 (0.86 GB, 2.0 TB/s;
 // 31 TFLOP/s).  128 threads with 8 x 4 outputs each were slower (161 against 139 us for 304: three CTAs
 // of four warps per SM do not cover the loads).
-template <typename T>
-constexpr size_t gj_update_smem() { return sizeof(cplx<T>) * kGjW * (64 + 64) + 2 * 64 * sizeof(int); }
+template <typename T, int TM, int TN>
+constexpr size_t gj_update_smem() {
+  return sizeof(cplx<T>) * kGjW * 16 * (TM + TN) + 16 * (TM + TN) * sizeof(int);
+}
 
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) k_gj_update(
+template <typename T, int TM, int TN>
+__global__ void __launch_bounds__(256, 3) k_gj_update(
     int n, int kb, int w, cplx<T>* A, int64_t lda, int64_t bsA, const cplx<T>* U, int64_t ldu, int64_t bsU,
     const int* __restrict__ piv, cplx<T>* out, int64_t ldo, int64_t bsO, int64_t boff) {
   using ct = cplx<T>;
   struct alignas(2 * sizeof(ct)) Pair { ct a, b; };
-  constexpr int BM = 64, BN = 64, TM = 4, TN = 4;
+  constexpr int BM = 16 * TM, BN = 16 * TN;
   extern __shared__ __align__(32) unsigned char dyn_gu[];
   ct* Us = reinterpret_cast<ct*>(dyn_gu);  // [w][BM]: the tile's rows of the pivot columns
   ct* Gs = Us + kGjW * BM;                 // [w][BN]
@@ -367,13 +370,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) k_gj_update(
   const int64_t b = blockIdx.z + boff;
   const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;  // rows ty + 16 i, columns 2 tx + (j & 1) + 32 (j >> 1)
+  const int tx = tid & 15, ty = tid >> 4;  // rows ty + 16 i
+  auto col = [&](int j) { return TN == 1 ? tx : 2 * tx + (j & 1) + 32 * (j >> 1); };
   ct* Ab = A + b * bsA;
   const int* pv = piv + b * n;
   const bool last = out != nullptr;
   if (tid < BN) col_k[tid] = -1;
-  for (int e = tid; e < w * 64; e += 256) {
-    const int c = e >> 6, i = e & 63;
+  static_assert(BM == BN, "one loop stages both tiles");
+  for (int e = tid; e < w * BM; e += 256) {
+    const int c = e / BM, i = e % BM;
     ct u = mk(T(0));
     if (row0 + i < n)
       u = last ? Ab[(int64_t)(row0 + i) * lda + pv[kb + c]] : U[b * bsU + (int64_t)c * ldu + row0 + i];
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) k_gj_update(
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int r = row0 + ty + 16 * i, c = col0 + 2 * tx + (j & 1) + 32 * (j >> 1);
+      const int r = row0 + ty + 16 * i, c = col0 + col(j);
       acc[i][j] = (r < n && c < n) ? Ab[(int64_t)r * lda + c] : mk(T(0));
     }
   if (last && tid < BM && row0 + tid < n) row_p[tid] = pv[row0 + tid];
@@ -397,7 +402,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) k_gj_update(
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < TN; ++j)
-    if (col_k[2 * tx + (j & 1) + 32 * (j >> 1)] >= kb) {  // a pivot column of this panel
+    if (col_k[col(j)] >= kb) {  // a pivot column of this panel
 #pragma unroll
       for (int i = 0; i < TM; ++i) acc[i][j] = mk(T(0));
     }
@@ -406,11 +411,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) k_gj_update(
     ct u[TM], g[TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i) u[i] = Us[c * BM + ty + 16 * i];
+    if constexpr (TN == 1) {
+      g[0] = Gs[c * BN + tx];
+    } else {
 #pragma unroll
-    for (int j = 0; j < TN; j += 2) {
-      const Pair p = *reinterpret_cast<const Pair*>(Gs + c * BN + 2 * tx + 16 * j);
-      g[j] = p.a;
-      g[j + 1] = p.b;
+      for (int j = 0; j < TN; j += 2) {
+        const Pair p = *reinterpret_cast<const Pair*>(Gs + c * BN + 2 * tx + 16 * j);
+        g[j] = p.a;
+        g[j + 1] = p.b;
+      }
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i)
@@ -425,7 +434,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) k_gj_update(
     if (!last && panel) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int cl = 2 * tx + (j & 1) + 32 * (j >> 1), c = col0 + cl;
+      const int cl = col(j), c = col0 + cl;
       if (c >= n) continue;
       if (!last) {
         Ab[(int64_t)r * lda + c] = acc[i][j];
@@ -451,17 +460,21 @@ template <typename T>
 int inverse_panels(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Ainv, int64_t ldi, int64_t bsI,
                    int* piv, int* info, cudaStream_t s) {
   const int threads = (n + 31) / 32 * 32;
-  // panel width: 32 columns, fewer while the panel does not fit in shared memory
-  int w = kGjW;
+  // panel width: 32 rows in FP32, fewer while the panel does not fit in shared memory; 8 in FP64, where
+  // the panel's own n w^2 FMAs on one SM are its cost (one n = 98
+  // inverse: 1.10 ms with 32 rows, 0.45 with 8, 1.41 by the one-CTA LU before; n = 242: 3.7, 1.6 and 10.8)
+  int w = sizeof(T) == 4 ? kGjW : kGjSub;
   while (w > kGjSub && gj_panel_smem<T>(n, w, threads) > 200 * 1024) w -= kGjSub;
   w = std::min(w, n);
   const size_t psmem = gj_panel_smem<T>(n, w, threads);
-  constexpr size_t usmem = gj_update_smem<T>();
+  constexpr int TT = sizeof(T) == 4 ? 4 : 1;
+  constexpr size_t usmem = gj_update_smem<T, TT, TT>();
   auto panel = threads <= 512 ? k_gj_panel<T, 512> : k_gj_panel<T, 1024>;
+  auto update = k_gj_update<T, TT, TT>;
   if (cudaFuncSetAttribute(panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_gj_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usmem) != cudaSuccess)
+      cudaFuncSetAttribute(update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usmem) != cudaSuccess)
     return KHP_ERR_CUDA;
-  const int tiles = (n + 63) / 64;
+  const int tiles = (n + 16 * TT - 1) / (16 * TT);
   for (int kb = 0; kb < n; kb += w) {
     const int cw = std::min(w, n - kb);
     const bool last = kb + cw >= n;
@@ -470,7 +483,7 @@ int inverse_panels(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, c
                                                           info);
     for (int64_t off = 0; off < batch; off += kMaxGridY) {
       const unsigned nb = (unsigned)std::min<int64_t>(batch - off, kMaxGridY);
-      k_gj_update<T><<<dim3(tiles, tiles, nb), 256, usmem, s>>>(n, kb, cw, A, lda, bsA, Ainv, ldi, bsI, piv,
+      update<<<dim3(tiles, tiles, nb), 256, usmem, s>>>(n, kb, cw, A, lda, bsA, Ainv, ldi, bsI, piv,
                                                                last ? Ainv : nullptr, ldi, bsI, off);
       count_launches(1);
     }
@@ -504,7 +517,10 @@ int launch_inverse_blocked(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_
     }
   }
   if (n <= kGjMaxN) return inverse_panels<T>(batch, n, A, lda, bsA, Ainv, ldi, bsI, piv, info, s);
-  return launch_inverse_lu<T>(batch, n, A, lda, bsA, Ainv, ldi, bsI, piv, info, s);
+  // (beyond 12800 rows not even one panel column fits in shared memory)
+  if ((size_t)n * sizeof(cplx<T>) <= 200 * 1024)
+    return launch_inverse_lu<T>(batch, n, A, lda, bsA, Ainv, ldi, bsI, piv, info, s);
+  return launch_inverse<T>(batch, n, A, lda, bsA, Ainv, ldi, bsI, piv, info, s);
 }
 
 template int launch_inverse_blocked<double>(int64_t, int, cplx<double>*, int64_t, int64_t, cplx<double>*, int64_t,

@@ -468,23 +468,19 @@ __global__ void k_xrows(int64_t batch, int n, const cd* __restrict__ lam, const 
   }
 }
 
-// S = [[X1, X2], [X2, X1]] from the n x 2n solution [X1 | X2]
-__global__ void k_scatter_sym(int64_t batch, int n, const cd* __restrict__ X, cd* S, int* status) {
+// S = [[X1, X2], [X2, X1]]
+__global__ void k_scatter_sym(int64_t batch, int n, const cd* __restrict__ X1, const cd* __restrict__ X2, cd* S,
+                              int* status) {
   const int64_t nn = (int64_t)n * n;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < batch * 2 * nn; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = e / (2 * nn);
-    const int64_t rc = e % (2 * nn);
-    const int i = (int)(rc / (2 * n)), jj = (int)(rc % (2 * n));
-    const cd v = X[e];
-    cd* Sb = S + b * 4 * nn;
-    if (jj < n) {
-      Sb[(int64_t)i * n + jj] = v;
-      Sb[3 * nn + (int64_t)i * n + jj] = v;
-    } else {
-      Sb[nn + (int64_t)i * n + jj - n] = v;
-      Sb[2 * nn + (int64_t)i * n + jj - n] = v;
-    }
-    if (!cfinite(v)) status_or(status, b, KHP_BIT_NONFINITE);
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < batch * nn; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = e / nn, rc = e - b * nn;
+    const cd v1 = X1[e], v2 = X2[e];
+    cd* Sb = S + b * 4 * nn + rc;
+    Sb[0] = v1;
+    Sb[nn] = v2;
+    Sb[2 * nn] = v2;
+    Sb[3 * nn] = v1;
+    if (!cfinite(v1) || !cfinite(v2)) status_or(status, b, KHP_BIT_NONFINITE);
   }
 }
 
@@ -600,7 +596,7 @@ inline ModesWs plan_modes(Arena& a, int64_t batch, int nh) {
 }
 
 struct SmatWs {
-  cd *b0, *b1, *b2, *b3, *p1, *p2, *rhs, *tmp;
+  cd *b0, *b1, *b2, *b3, *p1, *p2, *r1, *r2, *tmp;
   int* piv;
 };
 inline SmatWs plan_smat(Arena& a, int64_t batch, int nh) {
@@ -612,7 +608,8 @@ inline SmatWs plan_smat(Arena& a, int64_t batch, int nh) {
   w.b3 = a.take<cd>(batch * nn);
   w.p1 = a.take<cd>(batch * nn);
   w.p2 = a.take<cd>(batch * nn);
-  w.rhs = a.take<cd>(batch * 2 * nn);
+  w.r1 = a.take<cd>(batch * nn);
+  w.r2 = a.take<cd>(batch * nn);
   w.tmp = a.take<cd>(batch * nn);
   w.piv = a.take<int>(batch * n);
   return w;
@@ -771,7 +768,7 @@ int khp_structure_prep(int64_t nmaps, int32_t nh, const double* conv, const doub
   const int64_t hh = (int64_t)nh * nh;
   const cd* C = (const cd*)conv;
   KHP_TRY(launch_copy<double>(nmaps, nh, nh, C, nh, hh, w.lu, nh, hh, s));
-  KHP_TRY(launch_inverse<double>(nmaps, nh, w.lu, nh, hh, (cd*)ic, nh, hh, w.piv, status, s));
+  KHP_TRY(launch_inverse_blocked<double>(nmaps, nh, w.lu, nh, hh, (cd*)ic, nh, hh, w.piv, status, s));
   k_row_scale_real<<<ew_grid(nmaps * hh), 256, 0, s>>>(nmaps, nh, gx, C, w.tmp);
   count_launches(1);
   KHP_TRY(launch_gemm<double>(nmaps, nh, nh, nh, mk(1.0), (const cd*)ic, nh, hh, w.tmp, nh, hh, mk(0.0), (cd*)hx, nh,
@@ -842,15 +839,15 @@ int khp_layer_smatrix(int64_t batch, int32_t nh, const double* W, const double* 
   const cd* L = (const cd*)lam;
   // t1 = W^-1 (W0 = I), t2 = V^-1 V0
   KHP_TRY(launch_copy<double>(batch, n, n, (const cd*)W, n, nn, w.b0, n, nn, s));
-  KHP_TRY(launch_inverse<double>(batch, n, w.b0, n, nn, w.b2, n, nn, w.piv, status, s));  // b2 = Wi
+  KHP_TRY(launch_inverse_blocked<double>(batch, n, w.b0, n, nn, w.b2, n, nn, w.piv, status, s));  // b2 = Wi
   KHP_TRY(launch_copy<double>(batch, n, n, (const cd*)V, n, nn, w.b1, n, nn, s));
-  KHP_TRY(launch_inverse<double>(batch, n, w.b1, n, nn, w.b3, n, nn, w.piv, status, s));  // b3 = Vi
+  KHP_TRY(launch_inverse_blocked<double>(batch, n, w.b1, n, nn, w.b3, n, nn, w.piv, status, s));  // b3 = Vi
   k_build_ab<<<ew_grid(batch * nn), 256, 0, s>>>(batch, nh, gx, gy, kp, k0, w.b2, w.b3, w.b0, w.b1);  // b0 = A, b1 = B
   KHP_TRY(cuda_status());
   count_launches(1);
   // Ai = A^-1 (b3 <- copy of A for the LU, b2 <- Ai)
   KHP_TRY(launch_copy<double>(batch, n, n, w.b0, n, nn, w.b3, n, nn, s));
-  KHP_TRY(launch_inverse<double>(batch, n, w.b3, n, nn, w.b2, n, nn, w.piv, status, s));
+  KHP_TRY(launch_inverse_blocked<double>(batch, n, w.b3, n, nn, w.b2, n, nn, w.piv, status, s));
   // p1 = X B Ai X
   KHP_TRY(launch_gemm<double>(batch, n, n, n, one, w.b1, n, nn, w.b2, n, nn, zero, w.p1, n, nn, s));
   k_xmx<<<ew_grid(batch * nn), 256, 0, s>>>(batch, n, L, depth, k0, w.p1);
@@ -858,19 +855,20 @@ int khp_layer_smatrix(int64_t batch, int32_t nh, const double* W, const double* 
   // p2 = T = A - p1 B
   KHP_TRY(launch_copy<double>(batch, n, n, w.b0, n, nn, w.p2, n, nn, s));
   KHP_TRY(launch_gemm<double>(batch, n, n, n, mone, w.p1, n, nn, w.b1, n, nn, one, w.p2, n, nn, s));
-  // rhs[:, :n] = p1 A - B
-  KHP_TRY(launch_copy<double>(batch, n, n, w.b1, n, nn, w.rhs, 2 * n, 2 * nn, s));
-  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, w.p1, n, nn, w.b0, n, nn, mone, w.rhs, 2 * n, 2 * nn, s));
-  // rhs[:, n:] = X (A - B Ai B)
+  // r1 = p1 A - B
+  KHP_TRY(launch_copy<double>(batch, n, n, w.b1, n, nn, w.r1, n, nn, s));
+  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, w.p1, n, nn, w.b0, n, nn, mone, w.r1, n, nn, s));
+  // r2 = X (A - B Ai B)
   KHP_TRY(launch_gemm<double>(batch, n, n, n, one, w.b2, n, nn, w.b1, n, nn, zero, w.b3, n, nn, s));  // b3 = Ai B
   KHP_TRY(launch_copy<double>(batch, n, n, w.b0, n, nn, w.tmp, n, nn, s));
   KHP_TRY(launch_gemm<double>(batch, n, n, n, mone, w.b1, n, nn, w.b3, n, nn, one, w.tmp, n, nn, s));
-  k_xrows<<<ew_grid(batch * nn), 256, 0, s>>>(batch, n, L, depth, k0, w.tmp, w.rhs + n, 2 * n, 2 * nn);
+  k_xrows<<<ew_grid(batch * nn), 256, 0, s>>>(batch, n, L, depth, k0, w.tmp, w.r2, n, nn);
   count_launches(1);
-  // [S11 | S12] = T^-1 rhs
-  KHP_TRY(launch_getrf<double>(batch, n, w.p2, n, nn, w.piv, status, s));
-  KHP_TRY(launch_getrs<double>(batch, n, w.p2, n, nn, w.piv, w.rhs, 2 * n, 2 * nn, 2 * n, s));
-  k_scatter_sym<<<ew_grid(batch * 2 * nn), 256, 0, s>>>(batch, n, w.rhs, (cd*)S, status);
+  // S11 = T^-1 r1, S12 = T^-1 r2 (b2 = T^-1)
+  KHP_TRY(launch_inverse_blocked<double>(batch, n, w.p2, n, nn, w.b2, n, nn, w.piv, status, s));
+  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, w.b2, n, nn, w.r1, n, nn, zero, w.b3, n, nn, s));
+  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, w.b2, n, nn, w.r2, n, nn, zero, w.tmp, n, nn, s));
+  k_scatter_sym<<<ew_grid(batch * nn), 256, 0, s>>>(batch, n, w.b3, w.tmp, (cd*)S, status);
   count_launches(1);
   return cuda_status();
 }
@@ -918,11 +916,13 @@ int khp_star_product(int64_t batch, int32_t n, const double* SA, int64_t sa_stri
   // D = I - SB11 SA22
   KHP_TRY(launch_identity<double>(batch, n, n, w.D, n, nn, one, s));
   KHP_TRY(launch_gemm<double>(batch, n, n, n, mone, B11, n, sb_stride, A22, n, sa_stride, one, w.D, n, nn, s));
-  KHP_TRY(launch_getrf<double>(batch, n, w.D, n, nn, w.piv, status, s));
-  // Y = D^-1 [SB11 SA21 | SB12]
-  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, B11, n, sb_stride, A21, n, sa_stride, zero, w.Y, 2 * n, 2 * nn, s));
-  KHP_TRY(launch_copy<double>(batch, n, n, B12, n, sb_stride, w.Y + n, 2 * n, 2 * nn, s));
-  KHP_TRY(launch_getrs<double>(batch, n, w.D, n, nn, w.piv, w.Y, 2 * n, 2 * nn, 2 * n, s));
+  // Y = D^-1 [SB11 SA21 | SB12] (D^-1 in the first half of U, which is written only after; D then holds
+  // SB11 SA21)
+  cd* Di = w.U;
+  KHP_TRY(launch_inverse_blocked<double>(batch, n, w.D, n, nn, Di, n, 2 * nn, w.piv, status, s));
+  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, B11, n, sb_stride, A21, n, sa_stride, zero, w.D, n, nn, s));
+  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, Di, n, 2 * nn, w.D, n, nn, zero, w.Y, 2 * n, 2 * nn, s));
+  KHP_TRY(launch_gemm<double>(batch, n, n, n, one, Di, n, 2 * nn, B12, n, sb_stride, zero, w.Y + n, 2 * n, 2 * nn, s));
   // S11 = SA11 + SA12 Y1 ; S12 = SA12 Y2
   KHP_TRY(launch_copy<double>(batch, n, n, A11, n, sa_stride, O, n, os, s));
   KHP_TRY(launch_gemm<double>(batch, n, n, n, one, A12, n, sa_stride, w.Y, 2 * n, 2 * nn, one, O, n, os, s));
