@@ -874,7 +874,18 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   // the blocked reduction keeps full 256-thread teams (its panel updates are parallel work; three
   // teams per SM already cover the SM), whatever team size suits the QR's serial window chase
   const int gthreads = blocked ? kTeamThreads : threads;
-  k_gehrd<T><<<(unsigned)batch, gthreads, smem, s>>>(n, A, lda, bsA, Z, blocked, only);
+  bool reduced = false;
+  if constexpr (sizeof(T) == 4) {
+    if (!only && gehrd_cluster_fits(batch, n)) {  // (the reflectors in W, free until the back-transform)
+      const int st = launch_gehrd_cluster(batch, n, A, lda, bsA, W, ldw, bsW, Z, s);
+      if (st) return st;
+      reduced = true;
+    }
+  }
+  if (!reduced) {
+    k_gehrd<T><<<(unsigned)batch, gthreads, smem, s>>>(n, A, lda, bsA, Z, blocked, only);
+    count_launches(1);
+  }
   // Z through the rotation log when the region holds at least one full sweep per matrix
   unsigned char* lg = nullptr;
   if (logbuf && !only && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
@@ -882,7 +893,7 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
     lg = static_cast<unsigned char*>(logbuf);
   const size_t ssm = schur_smem<T>(n, lg != nullptr);
   if (ssm > 40 * 1024 &&
-      cudaFuncSetAttribute(k_geev_schur<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm) != cudaSuccess)
+      cudaFuncSetAttribute(k_geev_schur<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
     return KHP_ERR_CUDA;
   // FP32: a warp for the chase and, up to 288 threads, one per strip; fewer strips than threads still
   // gain (eigenvectors of the triangular factor): n = 50, 151 matrices: 128 threads 781 us, 256 626;
@@ -895,7 +906,7 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
                                              : kTeamThreads + 32;
   k_geev_schur<T><<<(unsigned)batch, sthreads, ssm, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes,
                                                        only);
-  count_launches(2);
+  count_launches(1);
   int st = cuda_status();
   if (st) return st;
   if (lg) {

@@ -455,6 +455,7 @@ void inv_reg(int64_t batch, int n, const cplx<float>* A, int64_t lda, int64_t bs
 
 // Largest n of the panel form: a thread per column.
 constexpr int kGjMaxN = 1024;
+constexpr int kGjPanelSmem = 200 * 1024;
 
 template <typename T>
 int inverse_panels(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Ainv, int64_t ldi, int64_t bsI,
@@ -464,14 +465,14 @@ int inverse_panels(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, c
   // the panel's own n w^2 FMAs on one SM are its cost (one n = 98
   // inverse: 1.10 ms with 32 rows, 0.45 with 8, 1.41 by the one-CTA LU before; n = 242: 3.7, 1.6 and 10.8)
   int w = sizeof(T) == 4 ? kGjW : kGjSub;
-  while (w > kGjSub && gj_panel_smem<T>(n, w, threads) > 200 * 1024) w -= kGjSub;
+  while (w > kGjSub && gj_panel_smem<T>(n, w, threads) > (size_t)kGjPanelSmem) w -= kGjSub;
   w = std::min(w, n);
   const size_t psmem = gj_panel_smem<T>(n, w, threads);
   constexpr int TT = sizeof(T) == 4 ? 4 : 1;
   constexpr size_t usmem = gj_update_smem<T, TT, TT>();
   auto panel = threads <= 512 ? k_gj_panel<T, 512> : k_gj_panel<T, 1024>;
   auto update = k_gj_update<T, TT, TT>;
-  if (cudaFuncSetAttribute(panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem) != cudaSuccess ||
+  if (cudaFuncSetAttribute(panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjPanelSmem) != cudaSuccess ||
       cudaFuncSetAttribute(update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usmem) != cudaSuccess)
     return KHP_ERR_CUDA;
   const int tiles = (n + 16 * TT - 1) / (16 * TT);

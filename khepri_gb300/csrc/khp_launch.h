@@ -35,6 +35,12 @@ template <typename T>
 int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z, cplx<T>* W, int64_t ldw,
                 int64_t bsW, cplx<T>* lam, int64_t bsLam, int* info, cudaStream_t s, void* logbuf = nullptr,
                 int64_t log_bytes = 0, const int* only = nullptr);
+// Hessenberg form of FP32 matrices in the shared memory of clusters (A becomes H, Z = Q; V: n x n
+// scratch per matrix, left with the reflectors); gehrd_cluster_fits: whether n fits and the batch
+// gains.
+bool gehrd_cluster_fits(int64_t batch, int n);
+int launch_gehrd_cluster(int64_t batch, int n, cplx<float>* A, int64_t lda, int64_t bsA, cplx<float>* V, int64_t ldv,
+                         int64_t bsV, cplx<float>* Z, cudaStream_t s);
 // Columns of W to unit 2-norm.
 template <typename T>
 int launch_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW, cudaStream_t s,

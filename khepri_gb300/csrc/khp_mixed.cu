@@ -314,7 +314,7 @@ int launch_clusters(int64_t batch, int n, const cd* mu, const cf* E, int* lab, i
   const int in_smem = cluster_smem(n) <= 200 * 1024 ? 1 : 0;  // (larger n: the label arrays in global memory)
   const size_t smem = in_smem ? cluster_smem(n) : kClusterWarps;
   if (smem > 40 * 1024 &&
-      cudaFuncSetAttribute(k_clusters, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      cudaFuncSetAttribute(k_clusters, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
     return KHP_ERR_CUDA;
   k_clusters<<<(unsigned)batch, kClusterThreads, smem, s>>>(n, mu, E, lab, pos, csz, memb, xc, mu_out, in_smem);
   count_launches(1);
