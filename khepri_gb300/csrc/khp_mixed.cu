@@ -63,13 +63,12 @@ __global__ void k_eig_residual(int64_t boff, int n, const cd* __restrict__ MW, c
   }
 }
 
-// The 2x2 eigen-decomposition of K = [[a, b], [c, d]] with eigenvectors scaled to unit
-// diagonal: returns den with v12 = -b/den, v21 = c/den, new eigenvalues a + bc/den and
-// d - bc/den (the root near a first).
-__device__ __forceinline__ cd pair_den(cd a, cd b, cd c, cd d) {
-  const cd h = 0.5 * (a - d);
-  const cd sq = csqrt(h * h + b * c);
-  return (h.re * sq.re + h.im * sq.im >= 0.0) ? h + sq : h - sq;
+// The 2x2 eigen-decomposition of K = [[a, b], [c, d]], h = (a - d) / 2, with eigenvectors scaled to
+// unit diagonal: returns den with v12 = -b/den, v21 = c/den, new eigenvalues a + bc/den and d - bc/den
+// (the root near a first).
+__device__ __forceinline__ cf pair_den(cf h, cf b, cf c) {
+  const cf sq = csqrt(h * h + b * c);
+  return (h.re * sq.re + h.im * sq.im >= 0.f) ? h + sq : h - sq;
 }
 
 // Eigenvalue clusters of the refinement: the connected components of the graph joining
@@ -100,17 +99,21 @@ struct ClusterWarp {
 // the similarity S^-1 K S with S = [[1, v12], [v21, 1]] on rows and columns (a, b), the 2x2 block's
 // eigenvectors scaled to unit diagonal, which zeroes K_ab and K_ba; X accumulates the S.  A sweep
 // takes the pairs in the rounds of a round-robin tournament: the k/2 disjoint pairs of a round are
-// rotated together, a lane per pair forming its rotation (FP64 square root and divisions, the cost of
-// a step), the lanes sharing the row and column updates.  Pairs degenerate within the noise, or
+// rotated together, a lane per pair forming its rotation, the lanes sharing the row and column updates.
+// v12 and v21 are formed in FP32: an FP64 square root and its divisions take ~500 instructions of a
+// pipe that starts one per 16 cycles and SM (20 us a pair, the cost of the whole kernel), and a v that is
+// 1e-7 off leaves 1e-7 of K_ab for the next sweep; the similarity itself, with 1/det refined to
+// FP64, is exact for the v that are used.  Pairs degenerate within the noise, or
 // whose S is nearly singular, are left alone and do not hold the sweeps up.  At most 16 sweeps,
 // stopping once every off-diagonal entry of the rotated pairs is below 1e-15 max|mu|.
 __device__ void cluster_jacobi(int k, ClusterWarp& w, double big) {
   const int lane = threadIdx.x & 31;
   for (int e = lane; e < k * k; e += 32) w.X[e] = mk(e / k == e % k ? 1.0 : 0.0);
   const int m = k + (k & 1), np = m / 2;
+  const double ibig = big > 0.0 ? 1.0 / big : 0.0;
   __syncwarp();
   for (int sweep = 0; sweep < 16; ++sweep) {
-    double off = 0.0;
+    float off = 0.f;
     for (int round = 0; round < m - 1; ++round) {
       if (lane < np) {
         int a = lane == 0 ? m - 1 : (round + lane) % (m - 1);
@@ -118,17 +121,26 @@ __device__ void cluster_jacobi(int k, ClusterWarp& w, double big) {
         if (a > b) { const int t = a; a = b; b = t; }
         int use = 0;
         if (b < k) {
-          const cd kab = w.K[a * k + b], kba = w.K[b * k + a];
-          const cd den = pair_den(w.K[a * k + a], kab, kba, w.K[b * k + b]);
-          if (cabs(den) > kDegenerateTol * big) {
-            const cd v12 = cdiv(mk(-kab.re, -kab.im), den), v21 = cdiv(kba, den);
-            const cd det = mk(1.0) - v12 * v21;
-            if (cabs(det) > 1e-3) {
+          // entries relative to max|mu|
+          const cd kab = w.K[a * k + b] * ibig, kba = w.K[b * k + a] * ibig;
+          const cd h = (w.K[a * k + a] - w.K[b * k + b]) * (0.5 * ibig);
+          const cf b32 = mk((float)kab.re, (float)kab.im), c32 = mk((float)kba.re, (float)kba.im);
+          const cf den = pair_den(mk((float)h.re, (float)h.im), b32, c32);
+          if (cabs(den) > (float)kDegenerateTol) {
+            const cf v12 = cdiv(-b32, den), v21 = cdiv(c32, den);
+            const cf det = mk(1.f) - v12 * v21;
+            if (cabs(det) > 1e-3f) {
               use = 1;
-              off = fmax(off, fmax(cabs(kab), cabs(kba)));
-              w.v12[lane] = v12;
-              w.v21[lane] = v21;
-              w.idet[lane] = cdiv(mk(1.0), det);
+              off = fmaxf(off, fmaxf(fmaxf(fabsf(b32.re), fabsf(b32.im)), fmaxf(fabsf(c32.re), fabsf(c32.im))));
+              const cd p = mk((double)v12.re, (double)v12.im), q = mk((double)v21.re, (double)v21.im);
+              const cd d64 = mk(1.0) - p * q;
+              const cf i32 = cdiv(mk(1.f), det);
+              cd id = mk((double)i32.re, (double)i32.im);
+#pragma unroll
+              for (int it = 0; it < 2; ++it) id = id * (mk(2.0) - d64 * id);  // Newton: 1e-7, 1e-14, FP64
+              w.v12[lane] = p;
+              w.v21[lane] = q;
+              w.idet[lane] = id;
               w.pb[lane] = b;
             }
           }
@@ -162,8 +174,8 @@ __device__ void cluster_jacobi(int k, ClusterWarp& w, double big) {
       }
       __syncwarp();
     }
-    for (int o = 16; o > 0; o >>= 1) off = fmax(off, __shfl_xor_sync(0xffffffffu, off, o));
-    if (off < 1e-15 * big) break;
+    for (int o = 16; o > 0; o >>= 1) off = fmaxf(off, __shfl_xor_sync(0xffffffffu, off, o));
+    if (off < 1e-15f) break;
   }
 }
 
@@ -181,10 +193,11 @@ constexpr size_t cluster_smem(int n) { return kClusterWarps + (size_t)n * (sizeo
 //
 // Bound by the dependent FP64 steps of the clusters' Jacobi sweeps (a warp per cluster) and by
 // the n^2 distances of every labelling pass, taken in FP32: an FP32 difference of eigenvalues is
-// within 3e-7 max|mu| of the FP64 one and the tolerances are at least 3.7e-5 max|mu|, so only pairs
-// within 10 % of a tolerance need FP64 to be decided as it would decide them.  Sweep of 151 symmetric
+// within 3e-7 max|mu| of the FP64 one, so only pairs that close to a tolerance (at least 3.7e-5
+// max|mu|) need FP64 to be decided as it would decide them.  Sweep of 151 symmetric
 // 5 x 5 problems 11.7 -> 9.9 ms, gradients of 32 9 x 9 problems 124 -> 102 ms against one thread per cluster
-// and FP64 distances.
+// and FP64 distances.  With the rotations in FP32 and the blocks shifted, 96 problems of 9 x 7
+// 3.45 -> 1.49 ms a call, the 32 of 9 x 9 7.9 -> 3.5.
 __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* __restrict__ mu,
                                                               const cf* __restrict__ E, int* lab, int* pos, int* csz,
                                                               int* memb, cf* xc, cd* mu_out, int in_smem) {
@@ -205,11 +218,12 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
   double big = 0.0;
   int bi = 0;
   for (int i = t.tid(); i < n; i += t.size()) {
-    big = fmax(big, cabs(m[i]));
+    big = fmax(big, norm2(m[i]));
     lb[i] = i;
     if (in_smem) mf[i] = make_float2((float)m[i].re, (float)m[i].im);
   }
   team_argmax(t, big, bi, &sh);
+  big = sqrt(big);
   double tol = kClusterTol * big;
   for (int level = 0; level < kClusterLevels; ++level, tol *= (1.0 / 3.0)) {
     if (t.tid() == 0) changed = 0;
@@ -225,7 +239,8 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
     if (!changed) break;
     t.sync();
     const double tol2 = tol * tol;
-    const float lo2 = 0.9f * (float)tol2, hi2 = 1.1f * (float)tol2;
+    const float margin = (float)(1e-6 * big / tol) + 1e-6f;  // (of d2: twice that of d, rounded up)
+    const float lo2 = (1.f - margin) * (float)tol2, hi2 = (1.f + margin) * (float)tol2;
     const bool scaled = lo2 > 1e-30f && hi2 < 1e30f;  // FP32 squares in range
     auto close = [&](int i, int j) -> bool {
       if (in_smem && scaled) {
@@ -290,10 +305,13 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
         if (lb[j] == r) cw->mem[c++] = j;
     }
     __syncwarp();
+    // the block relative to its first eigenvalue: the sweeps then round at the cluster's spread, not at
+    // |mu|, and reach their stopping test (unshifted, a cluster near max|mu| made all 16 sweeps)
+    const cd m0 = m[cw->mem[0]];
     for (int e = lane; e < k * k; e += 32) {
       const int p = e / k, q = e - p * k;
       const cf v = Eb[(int64_t)cw->mem[p] * n + cw->mem[q]];
-      cw->K[e] = mk((double)v.re, (double)v.im) + (p == q ? m[cw->mem[p]] : mk(0.0));
+      cw->K[e] = mk((double)v.re, (double)v.im) + (p == q ? m[cw->mem[p]] - m0 : mk(0.0));
     }
     __syncwarp();
     cluster_jacobi(k, *cw, big);
@@ -301,7 +319,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
     for (int e = lane; e < k * k; e += 32) {
       const int q = e / k, p = e - q * k;  // column q of X, row p
       const int j = cw->mem[q];
-      if (p == 0) mu_out[b * n + j] = cw->K[q * k + q];
+      if (p == 0) mu_out[b * n + j] = cw->K[q * k + q] + m0;
       memb[(b * n + j) * kClusterMax + p] = cw->mem[p];
       xc[(b * n + j) * kClusterMax + p] = mk((float)cw->X[p * k + q].re, (float)cw->X[p * k + q].im);
     }
