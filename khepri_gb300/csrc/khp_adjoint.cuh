@@ -12,18 +12,41 @@
 // f2(mu) = mu^-1/2 (Daleckii-Krein), which stay finite for degenerate eigenvalues.
 #pragma once
 
-// y = A^T x for two columns; A row-major n x n, x, y [n][2]; accumulation in A's precision.
+// y = A^T x for two columns; A row-major n x n, x, y [n][2]; accumulation in A's precision.  A thread per
+// column, the rows split over groups of warps whose partial sums meet in part (kPartWarps x 64 entries of
+// shared memory).  Ends with a barrier.
 template <typename TA, typename TX, typename TY>
-__device__ void team_mvT2(const TeamCta& t, const cplx<TA>* A, int n, const cplx<TX>* x, cplx<TY>* y) {
-  for (int j = t.tid(); j < n; j += t.size()) {
+__device__ void team_mvT2(const TeamCta& t, const cplx<TA>* __restrict__ A, int n, const cplx<TX>* x,
+                          cplx<TY>* y, cplx<TA>* part) {
+  const int lane = t.tid() & 31, warp = t.tid() >> 5, nw = t.size() >> 5;
+  const int nblk = (n + 31) / 32, rg = max(1, nw / nblk), chunk = (n + rg - 1) / rg;
+  for (int w = warp; w < nblk * rg; w += nw) {
+    const int blk = w % nblk, r = w / nblk, j = blk * 32 + lane;
+    const int i1 = min(n, (r + 1) * chunk);
     cplx<TA> a0 = mk(TA(0)), a1 = mk(TA(0));
-    for (int i = 0; i < n; ++i) {
-      const cplx<TA> aij = A[(int64_t)i * n + j];
-      fma_acc(a0, aij, mk((TA)x[2 * i].re, (TA)x[2 * i].im));
-      fma_acc(a1, aij, mk((TA)x[2 * i + 1].re, (TA)x[2 * i + 1].im));
+    if (j < n)
+#pragma unroll 8
+      for (int i = r * chunk; i < i1; ++i) {
+        const cplx<TA> aij = A[(int64_t)i * n + j];
+        fma_acc(a0, aij, mk((TA)x[2 * i].re, (TA)x[2 * i].im));
+        fma_acc(a1, aij, mk((TA)x[2 * i + 1].re, (TA)x[2 * i + 1].im));
+      }
+    if (rg > 1) {
+      part[(w * 32 + lane) * 2] = a0;
+      part[(w * 32 + lane) * 2 + 1] = a1;
+    } else if (j < n) {
+      y[2 * j] = mk((TY)a0.re, (TY)a0.im);
+      y[2 * j + 1] = mk((TY)a1.re, (TY)a1.im);
     }
-    y[2 * j] = mk((TY)a0.re, (TY)a0.im);
-    y[2 * j + 1] = mk((TY)a1.re, (TY)a1.im);
+  }
+  t.sync();
+  if (rg > 1) {
+    for (int e = t.tid(); e < 2 * n; e += t.size()) {
+      cplx<TA> v = mk(TA(0));
+      for (int r = 0; r < rg; ++r) v += part[r * nblk * 64 + e];
+      y[e] = mk((TY)v.re, (TY)v.im);
+    }
+    t.sync();
   }
 }
 
@@ -121,11 +144,14 @@ __global__ void __launch_bounds__(128) k_flux_grad(int nh, int npol, const cd* _
 // ------------------------------------------------------------------------------------------
 // RHO = F^T y - g in the layout of the unknowns (X, XA, RT), FP64.  Y in the residual layout.
 // ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_stack_residual_T(Table tb, const double* gx, const double* gy,
-                                                          const double* kp, const double* k0v,
-                                                          const cd* __restrict__ Y, const cd* __restrict__ GR,
-                                                          const cd* __restrict__ GT, cd* RX, cd* RXA, cd* RRT,
-                                                          cd* scratch) {
+// y_zero: Y is zero (the first round), so are the layers' products.  use_df: the products in double-float
+// on the FP32 pipe (as k_stack_residual; the FP64 pipe's 8 FMAs per element bound them otherwise), with
+// their operands as pairs in dfx ([batch][20 n] entries).
+__global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual_T(
+    Table tb, const double* gx, const double* gy, const double* kp, const double* k0v, const cd* __restrict__ Y,
+    const cd* __restrict__ GR, const cd* __restrict__ GT, cd* RX, cd* RXA, cd* RRT, cd* scratch, float4* dfx,
+    int y_zero, int use_df) {
+  __shared__ cd part[kPartWarps * 32 * 4];
   TeamCta t;
   const int64_t b = blockIdx.x;
   const int nh = tb.nh, n = 2 * nh, L = tb.L;
@@ -189,11 +215,21 @@ __global__ void __launch_bounds__(256) k_stack_residual_T(Table tb, const double
     const double dk = E.dep.at(b) * k0;
     const cd* y3 = ys(l + 1, 2);
     const cd* y4 = ys(l + 1, 3);
-    team_mvT2(t, W, n, y1, p1);
-    team_mvT2(t, V, n, y2, p2);
-    team_mvT2(t, W, n, y3, p3);
-    team_mvT2(t, V, n, y4, p4);
-    t.sync();
+    if (y_zero) {
+      for (int e = t.tid(); e < 8 * n; e += t.size()) p1[e] = mk(0.0);  // p1 .. p4 are one block
+      t.sync();
+    } else if (use_df && M.W2) {
+      float4* f = dfx + b * 20 * n;
+      for (int e = t.tid(); e < 8 * n; e += t.size()) f[e] = df_of(y1[e]);  // y1 .. y4 are one block
+      t.sync();
+      team_mvT4_df(t, M.W2 + b * nn, n, f, f + 4 * n, p1, p3, part);
+      team_mvT4_df(t, M.V2 + b * nn, n, f + 2 * n, f + 6 * n, p2, p4, part);
+    } else {
+      team_mvT2(t, W, n, y1, p1, part);
+      team_mvT2(t, V, n, y2, p2, part);
+      team_mvT2(t, W, n, y3, p3, part);
+      team_mvT2(t, V, n, y4, p4, part);
+    }
     cd* rap = rxa + (2 * pl) * 2 * n;
     cd* ram = rxa + (2 * pl + 1) * 2 * n;
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
@@ -230,10 +266,11 @@ __global__ void __launch_bounds__(256) k_stack_residual_T(Table tb, const double
 // (residual -> correction).  Statements of k_stack_sweep in reverse order, each transposed.
 // Per-problem FP32 workspace [..][n][2]: s-bar at every gap (L+1), per layer 4 vectors, 8 temps.
 // ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* gx, const double* gy,
+__global__ void __launch_bounds__(32 * kPartWarps) k_stack_sweep_T(Table tb, const double* gx, const double* gy,
                                                        const double* kp, const double* k0v, const cd* __restrict__ RX,
                                                        const cd* __restrict__ RXA, const cd* __restrict__ RRT, cd* Y,
                                                        cf* WS) {
+  __shared__ cf part[kPartWarps * 32 * 2];
   TeamCta t;
   const int64_t b = blockIdx.x;
   const int nh = tb.nh, n = 2 * nh, L = tb.L;
@@ -283,7 +320,7 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
     // gap l+1: dcm = Gamma dcp + s ; both recorded
     for (int e = t.tid(); e < 2 * n; e += t.size()) T0[e] = to_f(rcm(l + 1)[e]);  // dcm-bar
     t.sync();
-    team_mvT2(t, gam(l + 1), n, T0, T1);
+    team_mvT2(t, gam(l + 1), n, T0, T1, part);
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       dp[e] = dp[e] + to_f(rcp(l + 1)[e]) + T1[e];
@@ -294,7 +331,7 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
       // dcp_{l+1} = inv1 (S21 dcp_l + w)
       const M2* S = E.blocks + b * nh * 4;
       cf* wb = LV(l, 0);
-      team_mvT2(t, E.inv1 + b * nn, n, dp, wb);
+      team_mvT2(t, E.inv1 + b * nn, n, dp, wb, part);
       t.sync();
       for (int e = t.tid(); e < 2 * n; e += t.size()) {
         const int i = e / 2, c = e % 2;
@@ -318,8 +355,8 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
       hb[e] = T0[e];
     }
     t.sync();
-    team_mvT2(t, E.zr + b * nn, n, T0, T1);    // (X a+)-bar from rho X a+
-    team_mvT2(t, E.inv1 + b * nn, n, dp, T2);  // T2-bar
+    team_mvT2(t, E.zr + b * nn, n, T0, T1, part);    // (X a+)-bar from rho X a+
+    team_mvT2(t, E.inv1 + b * nn, n, dp, T2, part);  // T2-bar
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       qb[e] = T2[e];
@@ -328,7 +365,7 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
       T3[e] = to_f(rap[e] + xi * xbar);  // a+-bar
     }
     t.sync();
-    team_mvT2(t, E.inv2 + b * nn, n, T3, T4);  // T3-bar
+    team_mvT2(t, E.inv2 + b * nn, n, T3, T4, part);  // T3-bar
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       dp[e] = mk(2.f, 0.f) * T4[e];
@@ -348,14 +385,14 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
       yA[e] += rr[e];
     }
     t.sync();
-    team_mvT2(t, gam(0), n, T0, T1);
+    team_mvT2(t, gam(0), n, T0, T1, part);
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       dp[e] = dp[e] + to_f(rcp(0)[e]) + T1[e];
       SB(0)[e] = SB(0)[e] + T0[e];
     }
     t.sync();
-    team_mvT2(t, tb.inv0 + b * nn, n, dp, T2);  // u
+    team_mvT2(t, tb.inv0 + b * nn, n, dp, T2, part);  // u
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       const int i = e / 2, c = e % 2;
@@ -380,7 +417,7 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
         T1[e] = to_f(blk_mvT(S, 1, nh, i, c, sl));  // T1-bar
       }
       t.sync();
-      team_mvT2(t, E.zr + b * nn, n, T1, T2);  // Z^T T1-bar
+      team_mvT2(t, E.zr + b * nn, n, T1, T2, part);  // Z^T T1-bar
       t.sync();
       for (int e = t.tid(); e < 2 * n; e += t.size()) T3[e] = wfwd[e] + T2[e];  // w-bar
       t.sync();
@@ -403,7 +440,7 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
     cf* qb = LV(l, 3);
     for (int e = t.tid(); e < 2 * n; e += t.size()) T0[e] = mk(0.5f, 0.f) * sl[e];
     t.sync();
-    team_mvT2(t, gam(l), n, T0, T1);  // T3-bar = 1/2 Gamma^T s-bar
+    team_mvT2(t, gam(l), n, T0, T1, part);  // T3-bar = 1/2 Gamma^T s-bar
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       k1b[e] = k1b[e] + T0[e] - T1[e];
@@ -420,8 +457,8 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
       T2[e] = to_f(z);
     }
     t.sync();
-    team_mvT2(t, M.V32 + b * nn, n, T2, T3);  // V^T z
-    team_mvT2(t, M.W32 + b * nn, n, k1b, T4);  // W^T k1-bar
+    team_mvT2(t, M.V32 + b * nn, n, T2, T3, part);  // V^T z
+    team_mvT2(t, M.W32 + b * nn, n, k1b, T4, part);  // W^T k1-bar
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       const cd xi = cexp(-(mk((double)lam[e / 2].re, (double)lam[e / 2].im) * dk));
@@ -430,7 +467,7 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
       T0[e] = mk(0.5f, 0.f) * hb[e];
     }
     t.sync();
-    team_mvT2(t, E.zr + b * nn, n, T0, T1);  // 1/2 rho^T h-bar
+    team_mvT2(t, E.zr + b * nn, n, T0, T1, part);  // 1/2 rho^T h-bar
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       const cf qv = qb[e] + T1[e];
@@ -438,8 +475,8 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
       T6[e] = mk(0.f) - T0[e] - qv;       // g4-bar = -1/2 h-bar - q-bar
     }
     t.sync();
-    team_mvT2(t, M.Wi + b * nn, n, T5, T2);  // T0-bar
-    team_mvT2(t, M.Vi + b * nn, n, T6, T3);  // T1-bar
+    team_mvT2(t, M.Wi + b * nn, n, T5, T2, part);  // T0-bar
+    team_mvT2(t, M.Vi + b * nn, n, T6, T3, part);  // T1-bar
     t.sync();
     for (int e = t.tid(); e < 2 * n; e += t.size()) {
       const int i = e / 2, c = e % 2;
@@ -470,8 +507,9 @@ __global__ void __launch_bounds__(256) k_stack_sweep_T(Table tb, const double* g
 //   u1 = W^T y1 + V^T y2, u3 = W^T y3 - V^T y4, v2 = V^T y2, v4 = V^T y4, w2, w4,
 //   s2 = w2 / lam, s4 = w4 / lam, z2 = W s2, z4 = W s4.
 // ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_layer_vectors(Table tb, int l, int pl, const double* k0v,
+__global__ void __launch_bounds__(32 * kPartWarps) k_layer_vectors(Table tb, int l, int pl, const double* k0v,
                                                        const cd* __restrict__ XA, const cd* __restrict__ Y, cd* VEC) {
+  __shared__ cd part[kPartWarps * 32 * 2];
   TeamCta t;
   const int64_t b = blockIdx.x;
   const int nh = tb.nh, n = 2 * nh, L = tb.L;
@@ -490,10 +528,10 @@ __global__ void __launch_bounds__(256) k_layer_vectors(Table tb, int l, int pl, 
   cd* v = VEC + b * 20 * n;
   cd *u1 = v, *u3 = v + 2 * n, *v2 = v + 4 * n, *v4 = v + 6 * n, *w2 = v + 8 * n, *w4 = v + 10 * n;
   cd *s2 = v + 12 * n, *s4 = v + 14 * n, *z2 = v + 16 * n, *z4 = v + 18 * n;
-  team_mvT2(t, W, n, y1, u1);
-  team_mvT2(t, V, n, y2, v2);
-  team_mvT2(t, W, n, y3, u3);
-  team_mvT2(t, V, n, y4, v4);
+  team_mvT2(t, W, n, y1, u1, part);
+  team_mvT2(t, V, n, y2, v2, part);
+  team_mvT2(t, W, n, y3, u3, part);
+  team_mvT2(t, V, n, y4, v4, part);
   for (int e = t.tid(); e < 2 * n; e += t.size()) {
     const cd xi = xprop(lam, e / 2, dk);
     const cd a = xi * am[e] - ap[e], c = am[e] - xi * ap[e];

@@ -541,29 +541,89 @@ __device__ __forceinline__ void df_mac(float& sh, float& sl, float ah, float al,
   sl += err + e;
 }
 
-// y = A x for two columns, A row-major n x n as double-float pairs, x [n][2] as double-float
-// pairs, y [n][2] FP64 (hi + lo of each accumulator).  A thread per row; x is read by every
-// thread in the same order (broadcast loads).
-__device__ void team_mv2_df(const TeamCta& t, const float4* __restrict__ A, int n, const float4* __restrict__ x,
-                            cd* y) {
-  for (int i = t.tid(); i < n; i += t.size()) {
-    float r0h = 0.f, r0l = 0.f, i0h = 0.f, i0l = 0.f, r1h = 0.f, r1l = 0.f, i1h = 0.f, i1l = 0.f;
-    const float4* row = A + (int64_t)i * n;
-    for (int j = 0; j < n; ++j) {
+// (Products of a CTA with two or four columns.  Four lanes share a row: 64 bytes of it per load and lane
+// group instead of 16 bytes of 32 rows, and small matrices keep all threads busy; their partial sums
+// meet by shuffle.  Bound by the loads in flight: 912 problems of n = 98, one sweep, 2.20 -> 1.39 ms against
+// a thread per row, 912 of n = 242 5.93 -> 5.46.)
+//
+// ya = A xa and yb = A xb for two columns each; A row-major n x n as double-float pairs, xa, xb [n][2] as
+// double-float pairs, ya, yb [n][2] FP64 (hi + lo of each accumulator); A is read once for both.
+__device__ void team_mv4_df(const TeamCta& t, const float4* __restrict__ A, int n, const float4* xa,
+                            const float4* xb, cd* ya, cd* yb) {
+  const int sub = t.tid() & 3, grp = t.tid() >> 2, ng = t.size() >> 2;
+  for (int i0 = 0; i0 < n; i0 += ng) {
+    const int i = i0 + grp;
+    const float4* row = A + (int64_t)min(i, n - 1) * n;
+    float rh[4], rl[4], ih[4], il[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) rh[c] = rl[c] = ih[c] = il[c] = 0.f;
+#pragma unroll 2
+    for (int j = sub; j < n; j += 4) {
       const float4 a = row[j];
-      const float4 u = x[2 * j], v = x[2 * j + 1];
-      // (a.x + i a.y) + (a.z + i a.w) times (u.x + i u.y) + (u.z + i u.w), column 0
-      df_mac(r0h, r0l, a.x, a.z, u.x, u.z);
-      df_mac(r0h, r0l, -a.y, -a.w, u.y, u.w);
-      df_mac(i0h, i0l, a.x, a.z, u.y, u.w);
-      df_mac(i0h, i0l, a.y, a.w, u.x, u.z);
-      df_mac(r1h, r1l, a.x, a.z, v.x, v.z);
-      df_mac(r1h, r1l, -a.y, -a.w, v.y, v.w);
-      df_mac(i1h, i1l, a.x, a.z, v.y, v.w);
-      df_mac(i1h, i1l, a.y, a.w, v.x, v.z);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float4 u = c < 2 ? xa[2 * j + c] : xb[2 * j + c - 2];
+        // (a.x + i a.y) + (a.z + i a.w) times (u.x + i u.y) + (u.z + i u.w)
+        df_mac(rh[c], rl[c], a.x, a.z, u.x, u.z);
+        df_mac(rh[c], rl[c], -a.y, -a.w, u.y, u.w);
+        df_mac(ih[c], il[c], a.x, a.z, u.y, u.w);
+        df_mac(ih[c], il[c], a.y, a.w, u.x, u.z);
+      }
     }
-    y[2 * i] = mk((double)r0h + (double)r0l, (double)i0h + (double)i0l);
-    y[2 * i + 1] = mk((double)r1h + (double)r1l, (double)i1h + (double)i1l);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      double re = (double)rh[c] + (double)rl[c], im = (double)ih[c] + (double)il[c];
+      for (int o = 1; o < 4; o <<= 1) {
+        re += __shfl_xor_sync(0xffffffffu, re, o);
+        im += __shfl_xor_sync(0xffffffffu, im, o);
+      }
+      if (i < n && sub == c) (c < 2 ? ya : yb)[2 * i + (c & 1)] = mk(re, im);
+    }
+  }
+}
+
+// ya = A^T xa and yb = A^T xb, as team_mv4_df; a thread per column, the rows split over groups of warps
+// whose partial sums meet in part (kPartWarps x 128 entries of shared memory).  Ends with a barrier.
+constexpr int kPartWarps = 16;  // warps of the largest team
+__device__ void team_mvT4_df(const TeamCta& t, const float4* __restrict__ A, int n, const float4* xa,
+                             const float4* xb, cd* ya, cd* yb, cd* part) {
+  const int lane = t.tid() & 31, warp = t.tid() >> 5, nw = t.size() >> 5;
+  const int nblk = (n + 31) / 32, rg = max(1, nw / nblk), chunk = (n + rg - 1) / rg;
+  for (int w = warp; w < nblk * rg; w += nw) {
+    const int blk = w % nblk, r = w / nblk, j = blk * 32 + lane;
+    const int i1 = min(n, (r + 1) * chunk);
+    float rh[4], rl[4], ih[4], il[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) rh[c] = rl[c] = ih[c] = il[c] = 0.f;
+    if (j < n)
+#pragma unroll 4
+      for (int i = r * chunk; i < i1; ++i) {
+        const float4 a = A[(int64_t)i * n + j];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float4 u = c < 2 ? xa[2 * i + c] : xb[2 * i + c - 2];
+          df_mac(rh[c], rl[c], a.x, a.z, u.x, u.z);
+          df_mac(rh[c], rl[c], -a.y, -a.w, u.y, u.w);
+          df_mac(ih[c], il[c], a.x, a.z, u.y, u.w);
+          df_mac(ih[c], il[c], a.y, a.w, u.x, u.z);
+        }
+      }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const cd v = mk((double)rh[c] + (double)rl[c], (double)ih[c] + (double)il[c]);
+      if (rg > 1) part[(w * 32 + lane) * 4 + c] = v;
+      else if (j < n) (c < 2 ? ya : yb)[2 * j + (c & 1)] = v;
+    }
+  }
+  t.sync();
+  if (rg > 1) {
+    for (int e = t.tid(); e < 4 * n; e += t.size()) {
+      const int j = e >> 2, c = e & 3;
+      cd v = mk(0.0);
+      for (int r = 0; r < rg; ++r) v += part[(r * nblk * 32 + j) * 4 + c];
+      (c < 2 ? ya : yb)[2 * j + (c & 1)] = v;
+    }
+    t.sync();
   }
 }
 
@@ -622,42 +682,49 @@ __device__ __forceinline__ cd ld2(const V* v, int i, int c) {
   return mk((double)v[2 * i + c].re, (double)v[2 * i + c].im);
 }
 
-// y = A x for two columns; A row-major n x n, x, y [n][2]; accumulation in A's precision.  A
-// thread per row.  FP32 A with n even (n = 2 nh here): two elements per 16-byte load (row
-// starts are 16-byte aligned since n is even and the matrices 256-byte aligned), which halves the
-// L1 requests of these row-strided loads.
+// y = A x for two columns; A row-major n x n, x, y [n][2]; accumulation in A's precision.  Four lanes per
+// row; FP32 with n even (n = 2 nh here): two elements per 16-byte load (row starts are 16-byte aligned
+// since n is even and the matrices 256-byte aligned).
 template <typename TA, typename TX, typename TY>
-__device__ void team_mv2(const TeamCta& t, const cplx<TA>* A, int n, const cplx<TX>* x, cplx<TY>* y) {
-  if constexpr (sizeof(TA) == 4) {
-    if ((n & 1) == 0) {
-      for (int i = t.tid(); i < n; i += t.size()) {
-        cplx<TA> a0 = mk(TA(0)), a1 = mk(TA(0));
-        const float4* row = reinterpret_cast<const float4*>(A + (int64_t)i * n);
-        for (int j2 = 0; j2 < n / 2; ++j2) {
-          const float4 v = row[j2];
-          const int j = 2 * j2;
-          const cplx<TA> p = mk(v.x, v.y), q = mk(v.z, v.w);
-          fma_acc(a0, p, mk((TA)x[2 * j].re, (TA)x[2 * j].im));
-          fma_acc(a1, p, mk((TA)x[2 * j + 1].re, (TA)x[2 * j + 1].im));
-          fma_acc(a0, q, mk((TA)x[2 * j + 2].re, (TA)x[2 * j + 2].im));
-          fma_acc(a1, q, mk((TA)x[2 * j + 3].re, (TA)x[2 * j + 3].im));
-        }
-        y[2 * i] = mk((TY)a0.re, (TY)a0.im);
-        y[2 * i + 1] = mk((TY)a1.re, (TY)a1.im);
-      }
-      return;
-    }
-  }
-  for (int i = t.tid(); i < n; i += t.size()) {
+__device__ void team_mv2(const TeamCta& t, const cplx<TA>* __restrict__ A, int n, const cplx<TX>* x,
+                         cplx<TY>* y) {
+  const int sub = t.tid() & 3, grp = t.tid() >> 2, ng = t.size() >> 2;
+  for (int i0 = 0; i0 < n; i0 += ng) {
+    const int i = i0 + grp;
+    const cplx<TA>* row = A + (int64_t)min(i, n - 1) * n;
     cplx<TA> a0 = mk(TA(0)), a1 = mk(TA(0));
-    const cplx<TA>* row = A + (int64_t)i * n;
-    for (int j = 0; j < n; ++j) {
-      const cplx<TA> aij = row[j];
-      fma_acc(a0, aij, mk((TA)x[2 * j].re, (TA)x[2 * j].im));
-      fma_acc(a1, aij, mk((TA)x[2 * j + 1].re, (TA)x[2 * j + 1].im));
+    bool paired = false;
+    if constexpr (sizeof(TA) == 4) paired = (n & 1) == 0;
+    if (paired) {
+      if constexpr (sizeof(TA) == 4) {
+        const float4* r4 = reinterpret_cast<const float4*>(row);
+#pragma unroll 4
+        for (int j2 = sub; j2 < n / 2; j2 += 4) {
+          const float4 v = r4[j2];
+          const cplx<TA> p = mk(v.x, v.y), q = mk(v.z, v.w);
+          const cplx<TX>* xj = x + 4 * j2;
+          fma_acc(a0, p, mk((TA)xj[0].re, (TA)xj[0].im));
+          fma_acc(a1, p, mk((TA)xj[1].re, (TA)xj[1].im));
+          fma_acc(a0, q, mk((TA)xj[2].re, (TA)xj[2].im));
+          fma_acc(a1, q, mk((TA)xj[3].re, (TA)xj[3].im));
+        }
+      }
+    } else {
+#pragma unroll 4
+      for (int j = sub; j < n; j += 4) {
+        const cplx<TA> aij = row[j];
+        fma_acc(a0, aij, mk((TA)x[2 * j].re, (TA)x[2 * j].im));
+        fma_acc(a1, aij, mk((TA)x[2 * j + 1].re, (TA)x[2 * j + 1].im));
+      }
     }
-    y[2 * i] = mk((TY)a0.re, (TY)a0.im);
-    y[2 * i + 1] = mk((TY)a1.re, (TY)a1.im);
+    for (int o = 1; o < 4; o <<= 1) {
+      a0.re += __shfl_xor_sync(0xffffffffu, a0.re, o);
+      a0.im += __shfl_xor_sync(0xffffffffu, a0.im, o);
+      a1.re += __shfl_xor_sync(0xffffffffu, a1.re, o);
+      a1.im += __shfl_xor_sync(0xffffffffu, a1.im, o);
+    }
+    if (i < n && sub == 0) y[2 * i] = mk((TY)a0.re, (TY)a0.im);
+    if (i < n && sub == 1) y[2 * i + 1] = mk((TY)a1.re, (TY)a1.im);
   }
 }
 
@@ -677,7 +744,7 @@ __device__ __forceinline__ cd src_col(const M2* S, int q, int nh, int i, int c) 
 __device__ __forceinline__ cd xprop(const cd* lam64, int i, double dk) { return cexp(-(lam64[i] * dk)); }
 
 // FP64 residual of the stack equations at the current unknowns x (see the Elem comments).
-__global__ void __launch_bounds__(256) k_stack_residual(Table tb, const double* gx, const double* gy,
+__global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual(Table tb, const double* gx, const double* gy,
                                                         const double* kp, const double* k0v, const cd* __restrict__ X,
                                                         const cd* __restrict__ XA, const cd* __restrict__ RT,
                                                         cd* RES, cd* scratch, const int* active, int x_zero,
@@ -766,10 +833,8 @@ __global__ void __launch_bounds__(256) k_stack_residual(Table tb, const double* 
       t.sync();
       const float4* W2 = M.W2 + b * nn;
       const float4* V2 = M.V2 + b * nn;
-      team_mv2_df(t, W2, n, f1, r1);
-      team_mv2_df(t, V2, n, f2, r2);
-      team_mv2_df(t, W2, n, f3, r3);
-      team_mv2_df(t, V2, n, f4, r4);
+      team_mv4_df(t, W2, n, f1, f3, r1, r3);
+      team_mv4_df(t, V2, n, f2, f4, r2, r4);
     } else {
       for (int e = t.tid(); e < 2 * n; e += t.size()) {
         const cd xi = xprop(lam, e / 2, dk);
@@ -815,7 +880,7 @@ __global__ void __launch_bounds__(256) k_stack_residual(Table tb, const double* 
 // FP32 affine sweep: solves the stack equations for the residual RES (correction system) with
 // the kept factors, and adds the correction to the FP64 unknowns.
 // Per problem workspace (FP32, [..][n][2]): s at every gap (L+1), per layer 5 vectors, 6 temps.
-__global__ void __launch_bounds__(256) k_stack_sweep(Table tb, const double* gx, const double* gy, const double* kp,
+__global__ void __launch_bounds__(32 * kPartWarps) k_stack_sweep(Table tb, const double* gx, const double* gy, const double* kp,
                                                      const double* k0v, const cd* __restrict__ RES, cd* X, cd* XA,
                                                      cd* RT, cf* WS, double* corr, const int* active) {
   __shared__ TeamShared sh;
@@ -1342,6 +1407,10 @@ GradPlan plan_grad(Arena& a, int64_t batch, int nh, int L, int64_t nmaps) {
   return g;
 }
 
+// Threads of the per-problem stack kernels: 512 while a problem has an SM to itself, else 256 (912
+// problems of n = 98 1.4 against 1.7 ms a call with 512).
+int stack_threads(int64_t batch) { return batch <= 2 * 152 ? 32 * kPartWarps : 256; }
+
 #define MX_TRY(x)        \
   do {                   \
     const int _s = (x);  \
@@ -1503,11 +1572,13 @@ int grad_mixed(const Table& tb, MixedPlan& p, GradPlan& g, const GradArgs& ga, i
   if (cudaMemsetAsync(g.Y, 0, sizeof(cd) * batch * (size_t)(L + 2) * 4 * 2 * n, s) != cudaSuccess)
     return KHP_ERR_CUDA;
   for (int it = 0; it < refine + 3; ++it) {
-    k_stack_residual_T<<<(unsigned)batch, 256, 0, s>>>(tb, gx, gy, kp, k0, g.Y, g.GR, g.GT, g.RX, g.RXA, g.RRT,
-                                                       g.scr4);
+    // (the products in double-float but for the last round, whose residual decides the accuracy)
+    k_stack_residual_T<<<(unsigned)batch, stack_threads(batch), 0, s>>>(
+        tb, gx, gy, kp, k0, g.Y, g.GR, g.GT, g.RX, g.RXA, g.RRT, g.scr4, reinterpret_cast<float4*>(g.VEC), it == 0,
+        it < refine + 2);
     count_launches(1);
     MX_TRY(cuda_status());
-    k_stack_sweep_T<<<(unsigned)batch, 256, 0, s>>>(tb, gx, gy, kp, k0, g.RX, g.RXA, g.RRT, g.Y, g.SWT);
+    k_stack_sweep_T<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, gx, gy, kp, k0, g.RX, g.RXA, g.RRT, g.Y, g.SWT);
     count_launches(1);
     MX_TRY(cuda_status());
   }
@@ -1538,7 +1609,7 @@ int grad_mixed(const Table& tb, MixedPlan& p, GradPlan& g, const GradArgs& ga, i
     for (int l = 0; l < L; ++l) {
       if (kinds[l] != 1) continue;
       if (slot[l] == (int)m) {
-        k_layer_vectors<<<(unsigned)batch, 256, 0, s>>>(tb, l, pl, k0, p.XA, g.Y, g.VEC);
+        k_layer_vectors<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, l, pl, k0, p.XA, g.Y, g.VEC);
         count_launches(1);
         MX_TRY(cuda_status());
         MX_EW(k_layer_accum, batch * nn, batch, n, p.lam64[m], depth_of(l), k0, p.XA, xas, pl, g.Y, ys_stride,
@@ -1775,11 +1846,11 @@ int solve_mixed(int64_t batch, int px, int py, int L, const int* kinds, const in
     // the refine rounds every problem runs take the products in double-float; the extra rounds
     // of the problems that have not converged by then (an ill-conditioned stack next to a Wood
     // anomaly, whose corrections stall at the double-float floor) take them in FP64
-    k_stack_residual<<<(unsigned)batch, 256, 0, s>>>(tb, gx, gy, kp, k0, p.X, p.XA, p.RT, p.RES, p.scr, act,
+    k_stack_residual<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, gx, gy, kp, k0, p.X, p.XA, p.RT, p.RES, p.scr, act,
                                                       it == 0 ? 1 : 0, it <= refine ? 1 : 0);
     count_launches(1);
     MX_TRY(cuda_status());
-    k_stack_sweep<<<(unsigned)batch, 256, 0, s>>>(tb, gx, gy, kp, k0, p.RES, p.X, p.XA, p.RT, p.SW,
+    k_stack_sweep<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, gx, gy, kp, k0, p.RES, p.X, p.XA, p.RT, p.SW,
                                                    p.corr + (it & 1) * batch, act);
     count_launches(1);
     MX_TRY(cuda_status());
