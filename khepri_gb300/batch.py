@@ -8,9 +8,11 @@ that share a pixmap share one eigensolve per problem.
 """
 from __future__ import annotations
 
+import collections
 import contextlib
 import ctypes
 import functools
+import time
 
 import numpy as np
 import torch
@@ -620,6 +622,31 @@ def _prep_args(wavelengths, kp, which, te, tm):
     return wl, P, kpa, which, te, tm
 
 
+def _group_cost(group):
+    """Relative device time of a shape group: a chunk's serial steps grow with n^2 while its matrices are
+    fewer than the SMs, then with their number."""
+    key, chunks = group
+    maps = max(1, len({s for kind, s in zip(key[1], key[2]) if kind == 1}))
+    n = 2 * key[0][0] * key[0][1]
+    return n * n * sum(1.0 + len(c) * maps / 152 for c in chunks)
+
+
+def _next_stream(events, wanted):
+    """Index of the stream to take the next chunk, of those ``wanted``: one with nothing in flight
+    (event None), else the first whose event is reached."""
+    ks = [k for k, w in enumerate(wanted) if w]
+    for k in ks:
+        if events[k] is None:
+            return k
+    if len(ks) == 1:
+        return ks[0]
+    while True:
+        for k in ks:
+            if events[k].query():
+                return k
+        time.sleep(2e-5)
+
+
 def solve_structures(structures, wavelengths, kp, which=None, te=1.0, tm=0.0, lattice="square", epsi=1.0,
                      epse=1.0, chunk=None, both_pols=False, method="mixed", refine=2, strict=True, device="cuda",
                      streams=4):
@@ -632,7 +659,7 @@ def solve_structures(structures, wavelengths, kp, which=None, te=1.0, tm=0.0, la
     prepared in one batched launch).  chunk: problems per call (None: the autotuned number of
     mode matrices per call for the group's size, divided by its maps per problem).
     method: "mixed" (default) or "gamma" (FP64).
-    streams: CUDA streams the shape groups are dealt to in turn, each stream with its own
+    streams: CUDA streams the shape groups are dealt to, longest first, each stream with its own
     workspaces; a group's chunks stay on its stream.  Many small groups (structures of uneven
     sizes) then fill the GPU together instead of one after the other; a chunk's flags are read
     (and its flagged problems re-solved) only when its stream takes its next chunk.
@@ -660,7 +687,7 @@ def solve_structures(structures, wavelengths, kp, which=None, te=1.0, tm=0.0, la
         """Repairs and results of the chunk in flight on stream k (on that stream)."""
         if pending[k] is None:
             return
-        idx, r, t, status, fix, keep = pending[k]
+        idx, r, t, status, fix, keep, done = pending[k]
         pending[k] = None
         with torch.cuda.stream(ss[k]):
             fix()
@@ -668,32 +695,41 @@ def solve_structures(structures, wavelengths, kp, which=None, te=1.0, tm=0.0, la
             T[idx] = t.cpu().numpy()
             st_all[idx] = status.cpu().numpy()
 
-    # a shape group's chunks run on one stream (they share the group's device data); groups are
-    # dealt to the streams in turn
+    # A shape group's chunks run on one stream (they share the group's device data).  Groups are taken
+    # longest first, each by the stream that runs dry first: a few large matrices keep a stream busy for
+    # tens of ms on a few SMs, and dealt in turn they queued behind one another while other streams had
+    # run dry (32 structures of 3 x 3 to 13 x 13 harmonics on 4 streams: 166 -> 129 ms).
     groups, digests = _group_plan(structures, which, chunk)
     lat = engine.lattice_vectors(lattice)
-    for gi, (key, chunk_idx) in enumerate(groups):
-        k = gi % K
-        struct_k = None
-        for idx in chunk_idx:
-            finish(k)  # the stream's workspaces are reused by its next chunk
-            with torch.cuda.stream(ss[k]):
-                if struct_k is None:
-                    struct_k = engine.StructureGPU(key[0], lat, dev)
-                _, _, plan, pmap, pdepth, _, _ = _chunk_item(structures, which, digests, key, idx, struct_k)
-                B = len(idx)
-                prob = engine.Problems.make(wl[idx], kpa[idx], te[idx], tm[idx], dev)
-                status = torch.zeros(B, dtype=torch.int32, device=dev)
-                # the autotuned chunk comes with its tuned eigensolver team size
-                with (autotune.tuned_team(struct_k.n) if chunk is None else contextlib.nullcontext()):
-                    if both_pols:
-                        tt, tmm = both_pol_weights(B, dev)
-                        r, t, fix = solve_chunk_gamma(struct_k, plan, prob, status, epsi, epse, tt, tmm, prec, refine,
-                                                      pmap, pdepth, defer_repair=True)
-                    else:
-                        r, t, fix = solve_chunk_gamma(struct_k, plan, prob, status, epsi, epse, precision=prec,
-                                                      refine=refine, pmap=pmap, pdepth=pdepth, defer_repair=True)
-                pending[k] = (idx, r, t, status, fix, (struct_k, plan, prob, pmap, pdepth))
+    todo = collections.deque(sorted(groups, key=_group_cost, reverse=True))
+    turn = [None] * K  # per stream: [struct, key, chunks left] of its group
+    while todo or any(turn):
+        k = _next_stream([p and p[-1] for p in pending], [bool(todo) or t is not None for t in turn])
+        finish(k)  # the stream's workspaces are reused by its next chunk
+        with torch.cuda.stream(ss[k]):
+            if turn[k] is None:
+                key, chunk_idx = todo.popleft()
+                turn[k] = [engine.StructureGPU(key[0], lat, dev), key, collections.deque(chunk_idx)]
+            struct_k, key, left = turn[k]
+            idx = left.popleft()
+            if not left:
+                turn[k] = None
+            _, _, plan, pmap, pdepth, _, _ = _chunk_item(structures, which, digests, key, idx, struct_k)
+            B = len(idx)
+            prob = engine.Problems.make(wl[idx], kpa[idx], te[idx], tm[idx], dev)
+            status = torch.zeros(B, dtype=torch.int32, device=dev)
+            # the autotuned chunk comes with its tuned eigensolver team size
+            with (autotune.tuned_team(struct_k.n) if chunk is None else contextlib.nullcontext()):
+                if both_pols:
+                    tt, tmm = both_pol_weights(B, dev)
+                    r, t, fix = solve_chunk_gamma(struct_k, plan, prob, status, epsi, epse, tt, tmm, prec, refine,
+                                                  pmap, pdepth, defer_repair=True)
+                else:
+                    r, t, fix = solve_chunk_gamma(struct_k, plan, prob, status, epsi, epse, precision=prec,
+                                                  refine=refine, pmap=pmap, pdepth=pdepth, defer_repair=True)
+            done = torch.cuda.Event()
+            done.record()
+        pending[k] = (idx, r, t, status, fix, (struct_k, plan, prob, pmap, pdepth), done)
     for k in range(K):
         finish(k)
     for s in ss[1:]:
