@@ -87,14 +87,14 @@ size_t schur_smem(int n, bool log) {
   return sizeof(HqrWindow<T>);
 }
 
-// Schur form of the Hessenberg matrix and eigenvectors of the triangular factor (X left in A,
-// Q in Z); the back-transform W = Z X runs afterwards as a batched tiled product.  With a log
+// Schur form of the Hessenberg matrix (T in A, Q in Z) and, with `vectors`, the eigenvectors of T (X in A);
+// the back-transform W = Z X runs afterwards as a batched tiled product.  With a log
 // region (log_bytes per matrix at logbuf) Z's updates are logged and left for k_hqr_apply_log.
 template <typename T>
 __global__ void __launch_bounds__(kTeamThreads + 32, sizeof(T) == 4 ? 2 : 1) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
                                                               cplx<T>* lam, int64_t bsLam, int* info,
                                                               unsigned char* logbuf, int64_t log_bytes,
-                                                              const int* __restrict__ only) {
+                                                              const int* __restrict__ only, int vectors) {
   __shared__ TeamShared ts;
   extern __shared__ __align__(16) unsigned char dyn[];  // schur_smem<T>
   TeamCta t;
@@ -116,8 +116,107 @@ __global__ void __launch_bounds__(kTeamThreads + 32, sizeof(T) == 4 ? 2 : 1) k_g
     HqrWindow<T>& hw = *reinterpret_cast<HqrWindow<T>*>(dyn);
     st = team_hqr_win(t, Ab, lda, n, Zb, n, hw.win, hw.rc, hw.rs, &ts);
   }
-  team_trevc(t, Ab, lda, n, lam + b * bsLam);
+  if (vectors) team_trevc(t, Ab, lda, n, lam + b * bsLam);
   if (threadIdx.x == 0 && st) info[b] |= st;
+}
+
+// Eigenvectors of the Schur factors, as team_trevc (same divisions, same order of every sum), 32 columns
+// per CTA: A's upper triangles -> X in the buffer W, unit upper triangular, and lam.
+//
+// Columns are independent, so a CTA keeps its 32 of X in shared memory, a column per lane.  From the
+// bottom, one warp solves a block of 16 rows in registers, then all warps take the block's products
+// out of the rows above it, 8 rows at a time (their 16 columns of A staged per warp).  Bound by the
+// divisions of the solves, n in a row.  In one CTA per matrix, as before, every row was two barriers
+// and an update of the whole triangle through L2: 5.7M cycles of the eigensolver's 29M for one n = 242.
+// One n = 242 eigensolver 12.7 -> 9.9 ms, 912 51.8 -> 45 ms, four n = 338 26 -> 20.9 ms (this kernel 0.1, 2 and 0.16).
+constexpr int kTrevcRows = 16, kTrevcWarps = 8;
+template <typename T>
+constexpr size_t trevc_smem(int n) {
+  return sizeof(cplx<T>) * ((size_t)32 * n + 32 * kTrevcRows + kTrevcRows * kTrevcRows + 8 * kTrevcWarps * kTrevcRows);
+}
+constexpr size_t kTrevcSmem = 220 * 1024;
+
+template <typename T>
+__global__ void __launch_bounds__(32 * kTrevcWarps) k_trevc(int n, const cplx<T>* __restrict__ A, int64_t lda,
+                                                            int64_t bsA, cplx<T>* X, int64_t ldx, int64_t bsX,
+                                                            cplx<T>* lam, int64_t bsLam, int64_t boff,
+                                                            const int* __restrict__ only) {
+  using ct = cplx<T>;
+  constexpr int R = kTrevcRows;
+  extern __shared__ __align__(16) unsigned char dyn_tv[];
+  ct* xs = reinterpret_cast<ct*>(dyn_tv);  // [n][32]
+  ct* xe = xs + (size_t)32 * n;            // [R][32]: the block's solved rows, 0 from each column's own row on
+  ct* td = xe + 32 * R;                    // [R][R]: A's diagonal block
+  ct* tr = td + R * R;                     // [warps][8][R]: rows above it
+  const int64_t b = blockIdx.y + boff;
+  if (only && !only[b]) return;
+  const ct* Ab = A + b * bsA;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c0 = 32 * ((int)gridDim.x - 1 - (int)blockIdx.x);  // (longest first)
+  const int k = c0 + lane, kc = min(k, n - 1);
+  const int top = min(n, c0 + 32);  // rows with nonzero entries
+  for (int i = warp; i < top; i += kTrevcWarps)
+    xs[32 * i + lane] = i < k ? -Ab[(int64_t)i * lda + kc] : mk(T(i == k ? 1 : 0));
+  const ct lk = Ab[(int64_t)kc * lda + kc];
+  if (warp == 0 && k < n) lam[b * bsLam + k] = lk;
+  const T smlnum = Eps<T>::safemin * (T(n) / Eps<T>::ulp);
+  const T smin = tmax(Eps<T>::ulp * abs1(lk), smlnum);
+  ct* tw = tr + 8 * R * warp;
+  for (int r0 = (top - 1) / R * R; r0 >= 0; r0 -= R) {
+    const int m = min(R, n - r0);
+    if (threadIdx.x < R * R) {
+      const int i = threadIdx.x / R, j = threadIdx.x % R;
+      td[threadIdx.x] = i < m && j < m ? Ab[(int64_t)(r0 + i) * lda + r0 + j] : mk(T(0));
+    }
+    __syncthreads();
+    if (warp == 0) {
+      ct x[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[i] = r0 + i < top ? xs[32 * (r0 + i) + lane] : mk(T(0));
+#pragma unroll
+      for (int j = R - 1; j >= 0; --j) {
+        ct e = mk(T(0));
+        if (r0 + j < k && r0 + j < top) {
+          ct den = td[j * R + j] - lk;
+          if (abs1(den) < smin) den = mk(smin);
+          x[j] = cdiv(x[j], den);
+          e = x[j];
+        }
+        xe[32 * j + lane] = e;
+#pragma unroll
+        for (int i = 0; i < j; ++i) fma_acc(x[i], -td[i * R + j], e);
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (r0 + i < top) xs[32 * (r0 + i) + lane] = x[i];
+    }
+    __syncthreads();
+    for (int i0 = 8 * warp; i0 < r0; i0 += 8 * kTrevcWarps) {  // (r0 is a multiple of 8)
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < 8 * R / 32; ++u) {
+        const int e = lane + 32 * u, i = e / R, j = e % R;
+        tw[e] = j < m ? -Ab[(int64_t)(i0 + i) * lda + r0 + j] : mk(T(0));
+      }
+      __syncwarp();
+      ct acc[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = xs[32 * (i0 + i) + lane];
+#pragma unroll
+      for (int j = R - 1; j >= 0; --j) {
+        const ct e = xe[32 * j + lane];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma_acc(acc[i], tw[i * R + j], e);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) xs[32 * (i0 + i) + lane] = acc[i];
+    }
+    __syncthreads();
+  }
+  if (k < n) {
+    ct* Xb = X + b * bsX;
+    for (int i = warp; i < n; i += kTrevcWarps) Xb[(int64_t)i * ldx + k] = i < top ? xs[32 * i + lane] : mk(T(0));
+  }
 }
 
 // The sweeps left in each matrix's rotation log applied to Z: a CTA of one warp holds
@@ -218,19 +317,32 @@ __global__ void __launch_bounds__(kLogRows) k_hqr_apply_log(int n, cplx<T>* Z, c
     for (int j = lane; j < n; j += kLogRows) Zb[(int64_t)(r0 + i) * n + j] = rows[i * lds + j];
 }
 
-// Scale every column of W to unit 2-norm (thread per column, coalesced along rows).
+// W = the columns of V at unit 2-norm; V may be W.  32 columns per CTA, the rows over 8 warps (a thread
+// per column took 75 us for one n = 242).
 template <typename T>
-__global__ void k_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW,
-                                 const int* __restrict__ only) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < batch * n; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = e / n;
+__global__ void __launch_bounds__(256) k_normalize_cols(int64_t batch, int n, const cplx<T>* V, int64_t ldv,
+                                                        int64_t bsV, cplx<T>* W, int64_t ldw, int64_t bsW,
+                                                        const int* __restrict__ only) {
+  __shared__ T part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cblk = (n + 31) / 32;
+  for (int64_t e = blockIdx.x; e < batch * cblk; e += gridDim.x) {
+    const int64_t b = e / cblk;
     if (only && !only[b]) continue;
-    const int k = (int)(e % n);
+    const int k = (int)(e % cblk) * 32 + lane;
+    const cplx<T>* v = V + b * bsV + k;
     cplx<T>* w = W + b * bsW + k;
     T s = T(0);
-    for (int i = 0; i < n; ++i) s += norm2(w[(int64_t)i * ldw]);
+    if (k < n)
+      for (int i = warp; i < n; i += 8) s += norm2(v[(int64_t)i * ldv]);
+    __syncthreads();
+    part[warp][lane] = s;
+    __syncthreads();
+    s = T(0);
+    for (int u = 0; u < 8; ++u) s += part[u][lane];
     const T inv = s > T(0) ? T(1) / sqrt(s) : T(1);
-    for (int i = 0; i < n; ++i) w[(int64_t)i * ldw] = w[(int64_t)i * ldw] * inv;
+    if (k < n)
+      for (int i = warp; i < n; i += 8) w[(int64_t)i * ldw] = v[(int64_t)i * ldv] * inv;
   }
 }
 
@@ -904,8 +1016,11 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
                        : n <= 32             ? 128
                        : n <= 224            ? kTeamThreads
                                              : kTeamThreads + 32;
+  // 32 columns of the eigenvectors fit in shared memory up to n = 849 (FP32), 425 (FP64)
+  const size_t tsm = trevc_smem<T>(n);
+  const bool columns = tsm <= kTrevcSmem;
   k_geev_schur<T><<<(unsigned)batch, sthreads, ssm, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes,
-                                                       only);
+                                                       only, columns ? 0 : 1);
   count_launches(1);
   int st = cuda_status();
   if (st) return st;
@@ -922,18 +1037,32 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
     st = cuda_status();
     if (st) return st;
   }
-  // W = Z X (X unit upper triangular, stored in A) and unit columns
+  // W = Z X (X unit upper triangular) and unit columns; X takes W's place and the product A's, or X is in A
+  if (columns) {
+    if (tsm > 40 * 1024 &&
+        cudaFuncSetAttribute(k_trevc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrevcSmem) != cudaSuccess)
+      return KHP_ERR_CUDA;
+    for (int64_t off = 0; off < batch; off += kMaxGridY) {
+      const unsigned nb = (unsigned)std::min<int64_t>(batch - off, kMaxGridY);
+      k_trevc<T><<<dim3((n + 31) / 32, nb), 32 * kTrevcWarps, tsm, s>>>(n, A, lda, bsA, W, ldw, bsW, lam, bsLam, off,
+                                                                        only);
+      count_launches(1);
+    }
+    st = launch_gemm<T>(batch, n, n, n, mk(T(1)), Z, n, (int64_t)n * n, W, ldw, bsW, mk(T(0)), A, lda, bsA, s, nullptr,
+                        nullptr, mk(T(0)), only);
+    return st ? st : launch_normalize_cols<T>(batch, n, A, lda, bsA, W, ldw, bsW, s, only);
+  }
   st = launch_gemm<T>(batch, n, n, n, mk(T(1)), Z, n, (int64_t)n * n, A, lda, bsA, mk(T(0)), W, ldw, bsW, s, nullptr,
                       nullptr, mk(T(0)), only);
-  return st ? st : launch_normalize_cols<T>(batch, n, W, ldw, bsW, s, only);
+  return st ? st : launch_normalize_cols<T>(batch, n, W, ldw, bsW, W, ldw, bsW, s, only);
 }
 
 template <typename T>
-int launch_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW, cudaStream_t s,
-                          const int* only) {
-  const int64_t cols = batch * n;
-  k_normalize_cols<T><<<(unsigned)std::min<int64_t>((cols + 127) / 128, 152 * 16), 128, 0, s>>>(batch, n, W, ldw, bsW,
-                                                                                               only);
+int launch_normalize_cols(int64_t batch, int n, const cplx<T>* V, int64_t ldv, int64_t bsV, cplx<T>* W, int64_t ldw,
+                          int64_t bsW, cudaStream_t s, const int* only) {
+  const int64_t blocks = batch * ((n + 31) / 32);
+  k_normalize_cols<T><<<(unsigned)std::min<int64_t>(blocks, 152 * 16), 256, 0, s>>>(batch, n, V, ldv, bsV, W, ldw, bsW,
+                                                                                    only);
   count_launches(1);
   return cuda_status();
 }
@@ -1164,7 +1293,8 @@ int launch_inverse_lu(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA
                               const int*, cplx<T>, const int*);                                                 \
   template int launch_geev<T>(int64_t, int, cplx<T>*, int64_t, int64_t, cplx<T>*, cplx<T>*, int64_t, int64_t,  \
                               cplx<T>*, int64_t, int*, cudaStream_t, void*, int64_t, const int*);               \
-  template int launch_normalize_cols<T>(int64_t, int, cplx<T>*, int64_t, int64_t, cudaStream_t, const int*);    \
+  template int launch_normalize_cols<T>(int64_t, int, const cplx<T>*, int64_t, int64_t, cplx<T>*, int64_t,      \
+                                        int64_t, cudaStream_t, const int*);                                     \
   template int launch_copy<T>(int64_t, int, int, const cplx<T>*, int64_t, int64_t, cplx<T>*, int64_t, int64_t,  \
                               cudaStream_t);                                                                    \
   template int launch_identity<T>(int64_t, int, int, cplx<T>*, int64_t, int64_t, cplx<T>, cudaStream_t);        \

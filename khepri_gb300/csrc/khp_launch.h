@@ -41,10 +41,10 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
 bool gehrd_cluster_fits(int64_t batch, int n);
 int launch_gehrd_cluster(int64_t batch, int n, cplx<float>* A, int64_t lda, int64_t bsA, cplx<float>* V, int64_t ldv,
                          int64_t bsV, cplx<float>* Z, cudaStream_t s);
-// Columns of W to unit 2-norm.
+// W = the columns of V at unit 2-norm (V may be W).
 template <typename T>
-int launch_normalize_cols(int64_t batch, int n, cplx<T>* W, int64_t ldw, int64_t bsW, cudaStream_t s,
-                          const int* only = nullptr);
+int launch_normalize_cols(int64_t batch, int n, const cplx<T>* V, int64_t ldv, int64_t bsV, cplx<T>* W, int64_t ldw,
+                          int64_t bsW, cudaStream_t s, const int* only = nullptr);
 
 // M W = W diag(lam) in FP64 (M [batch][n][n] destroyed; unit columns): FP32 eigensolver and FP64
 // refinement, the matrices whose residual test fails by the FP64 eigensolver (khp_mixed.cu).

@@ -1925,7 +1925,7 @@ int launch_geev_refined(int64_t batch, int n, cd* M, cd* W, cd* lam, int* info, 
   MX_TRY(launch_eig_check(batch, n, r.MW64, W, r.mu, nullptr, nullptr, mk(0.0), kRefinedTolPerN * n, 1, w.act, s));
   if (cudaMemcpyAsync(lam, r.mu, sizeof(cd) * batch * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return KHP_ERR_CUDA;
-  MX_TRY(launch_normalize_cols<double>(batch, n, W, n, nn, s));
+  MX_TRY(launch_normalize_cols<double>(batch, n, W, n, nn, W, n, nn, s));
   return launch_geev<double>(batch, n, M, n, nn, reinterpret_cast<cd*>(w.M32), W, n, nn, lam, n, info, s, nullptr, 0,
                              w.act);
 }
