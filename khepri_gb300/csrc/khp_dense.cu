@@ -90,8 +90,8 @@ size_t schur_smem(int n, bool log) {
 // Schur form of the Hessenberg matrix (T in A, Q in Z) and, with `vectors`, the eigenvectors of T (X in A);
 // the back-transform W = Z X runs afterwards as a batched tiled product.  With a log
 // region (log_bytes per matrix at logbuf) Z's updates are logged and left for k_hqr_apply_log.
-template <typename T>
-__global__ void __launch_bounds__(kTeamThreads + 32, sizeof(T) == 4 ? 2 : 1) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT, sizeof(T) == 4 && MAXT < 512 ? 2 : 1) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
                                                               cplx<T>* lam, int64_t bsLam, int* info,
                                                               unsigned char* logbuf, int64_t log_bytes,
                                                               const int* __restrict__ only, int vectors) {
@@ -1003,23 +1003,29 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   if (logbuf && !only && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
       hqr_log_view<T>(logbuf, log_bytes, n).cap_rot >= n - 1)
     lg = static_cast<unsigned char*>(logbuf);
+  // FP32: a warp for the chase, the others for the strips.  While a matrix has an SM to itself more threads
+  // than strips shorten their way to and from H (one n = 242: 256 threads 11.2 ms, 288 10.5, 352 9.4, 480
+  // 9.3; n = 162: 4.87, 4.83, 4.09, 4.15; n = 50: 557, 561, 542, 547 us).  Up to two matrices per SM two CTAs
+  // fit with 256 (304 of n = 98: 192 threads 2.67 ms, 256 2.41, 352 3.44).  Beyond, three of 192 where their
+  // shared memory fits (456 of n = 98: 192 threads 3.22, 256 4.48; of n = 150: 7.17, 8.87), else two of 288
+  // (456 of n = 162: 192 threads 13.8, 256 12.2, 288 11.0; of n = 242: 32.1, 29.5, 25.3).  Small matrices: 512
+  // of n = 18 with 128 threads 284 us, 160 270, 192 368.
+  const int sthreads = sizeof(T) == 8 || !lg           ? threads
+                       : eig_tuned(n) && batch > 152   ? std::max(64, threads)
+                       : n <= 32                       ? 160
+                       : batch <= 152                  ? (n <= 200 ? 352 : 480)
+                       : batch <= 2 * 152              ? kTeamThreads
+                       : n <= 150                      ? 192
+                                                       : kTeamThreads + 32;
+  auto schur = sthreads <= kTeamThreads + 32 ? k_geev_schur<T, kTeamThreads + 32> : k_geev_schur<T, 2 * kTeamThreads + 32>;
   const size_t ssm = schur_smem<T>(n, lg != nullptr);
   if (ssm > 40 * 1024 &&
-      cudaFuncSetAttribute(k_geev_schur<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
+      cudaFuncSetAttribute(schur, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
     return KHP_ERR_CUDA;
-  // FP32: a warp for the chase and, up to 288 threads, one per strip; fewer strips than threads still
-  // gain (eigenvectors of the triangular factor): n = 50, 151 matrices: 128 threads 781 us, 256 626;
-  // n = 98, 64: 160 threads 2.40 ms, 256 1.88; n = 242, 912: 256 threads 53.8 ms, 288 51.8; n = 18, 512:
-  // 128 threads 325 us, 256 425
-  const int sthreads = sizeof(T) == 8 || !lg ? threads
-                       : eig_tuned(n)        ? std::max(64, threads)
-                       : n <= 32             ? 128
-                       : n <= 224            ? kTeamThreads
-                                             : kTeamThreads + 32;
   // 32 columns of the eigenvectors fit in shared memory up to n = 849 (FP32), 425 (FP64)
   const size_t tsm = trevc_smem<T>(n);
   const bool columns = tsm <= kTrevcSmem;
-  k_geev_schur<T><<<(unsigned)batch, sthreads, ssm, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes,
+  schur<<<(unsigned)batch, sthreads, ssm, s>>>(n, A, lda, bsA, Z, lam, bsLam, info, lg, log_bytes,
                                                        only, columns ? 0 : 1);
   count_launches(1);
   int st = cuda_status();

@@ -171,9 +171,9 @@ __device__ __forceinline__ void hqr_chase(cplx<T>* win, HqrRot<T>* rot, int nrot
 // rolls its own copy of the next 31 columns' strips to complete the next window's first row.  One
 // CTA barrier per window.  Bound by the chase for a few matrices (n = 242: 48K rotations, 0.26 us each
 // with everything else) and by what a window moves between H and shared memory for many (two CTAs per
-// SM).  Schur form and eigenvectors, n = 50: 1.35 -> 0.60 ms, n = 98, 64 matrices: 3.9 -> 1.86, n = 242:
-// 31.0 -> 12.7, 912 matrices 89 (128 threads) -> 51.8, n = 578: 222 -> 107 (chase through shared memory
-// with three warp barriers a step, strips from global memory after it, before).
+// SM).  Against the chase through shared memory with three warp barriers a step and strips from global
+// memory after it (both with the triangular factor's eigenvectors): n = 50 1.35 -> 0.54 ms, n = 98,
+// 64 matrices 3.9 -> 1.74, n = 242 31.0 -> 9.3, 912 matrices 89 -> 43, n = 578 222 -> 72.
 template <typename T>
 __device__ __forceinline__ void cta_hqr_sweep(cplx<T>* H, int64_t ld, int n, int lo, int hi, cplx<T> mu,
                                               HqrShared<T>& sh, cplx<T>* strips, HqrRot<T>* log) {
