@@ -30,6 +30,29 @@ __device__ __forceinline__ unsigned pivot_key(cplx<double> v) {
   return x == 0.0 ? 1u : max((unsigned)__double2hiint(x), 1u) + 1u;
 }
 
+// 1/p for a pivot (nonzero): conj(p)/|p|^2 with p scaled by a power of two to a modulus of 1 to 2^1.5, one
+// division.  (khp_core.cuh's cdiv takes three divisions in a row and a branch, which every elimination
+// step waits for: in FP64, where a warp's instruction takes 16 cycles of the SM's pipe, 2.5 to 5K cycles of
+// a step's 5.3 to 9.6K.)  FP64 refines the FP32 reciprocal by two Newton steps (2^-22, 2^-44, rounding).
+__device__ __forceinline__ cplx<float> pivot_recip(cplx<float> p) {
+  const unsigned e = __float_as_uint(fmaxf(fabsf(p.re), fabsf(p.im))) >> 23;
+  const float sc = __uint_as_float((254u - min(e, 253u)) << 23);
+  const float x = p.re * sc, y = p.im * sc;
+  const float r = sc / (x * x + y * y);
+  return e < 255u ? mk(x * r, -y * r) : mk(0.f);  // (0 for an infinite pivot)
+}
+__device__ __forceinline__ cplx<double> pivot_recip(cplx<double> p) {
+  const int e = max(__double2hiint(fabs(p.re)), __double2hiint(fabs(p.im))) >> 20;
+  const double sc = __hiloint2double((2046 - min(e, 2045)) << 20, 0);
+  const double x = p.re * sc, y = p.im * sc;
+  const double d = x * x + y * y;
+  double r = (double)(1.0f / (float)d);
+  r = fma(r, fma(-d, r, 1.0), r);
+  r = fma(r, fma(-d, r, 1.0), r);
+  r *= sc;
+  return e < 2047 ? mk(x * r, -y * r) : mk(0.0);
+}
+
 // ------------------------------------------------------------------------------------------
 // Whole matrix in registers.  Warp w of NW holds rows w, w + NW, ..; lane l columns l, l + 32, ..:
 // element (w + NW j, l + 32 i) of the matrix in a[i][j].  Step k takes row k, picks the largest
@@ -89,7 +112,7 @@ __global__ void __launch_bounds__(32 * NW) k_inv_reg(int n, const cplx<float>* _
     const bool ok = best > 1u;  // 1: every candidate is 0; 0: every candidate is NaN
     if (!ok) st |= best == 1u ? KHP_BIT_SINGULAR : KHP_BIT_NONFINITE;
     if (lane == 0) {
-      pinv_s[buf] = ok ? cdiv(mk(1.f), pv) : mk(0.f);
+      pinv_s[buf] = ok ? pivot_recip(pv) : mk(0.f);
       pcol_s[buf] = ok ? p : ~p;  // ~p: the column is spent but nothing is eliminated
       pcol[k] = p;
       kinv[p] = k;
@@ -271,7 +294,7 @@ __global__ void __launch_bounds__(MAXT) k_gj_panel(int n, int kb, int w, cplx<T>
         ct* q = cand + (buf * nw + warp) * kGjSub;
 #pragma unroll
         for (int z = 0; z < kGjSub; ++z) q[z] = a[z];
-        if (best > 1u) cinv[buf * nw + warp] = cdiv(mk(T(1)), a[c]);
+        if (best > 1u) cinv[buf * nw + warp] = pivot_recip(a[c]);
       }
       if (lane == 0) {
         ckey[buf][warp] = best;
