@@ -7,6 +7,7 @@
 // Both leave the rows (columns) where they are: pivots are recorded, and the interchange of the
 // result's rows and columns happens as the inverse is written.
 #include <algorithm>
+#include <utility>
 
 #include "khepri_gb300.h"
 #include "khp_core.cuh"
@@ -219,8 +220,10 @@ __global__ void __launch_bounds__(32 * NW) k_inv_reg(int n, const cplx<float>* _
 // Panels of rows.  With P the pivot columns of a panel of rows J, D = A[J, P]: the panel becomes
 //   G[:, P] = D^-1,  G[:, j] = -D^-1 A[J, j] (other columns),
 // and every other row A[i, .] <- (P's columns 0, the others kept) + A[i, P] G.  k_gj_panel makes G in
-// place (scalar Gauss-Jordan steps, partial pivoting over the columns not yet used) and copies the
-// pivot columns' old values aside; k_gj_update applies it.  (Pivots are searched along rows because
+// place (scalar Gauss-Jordan steps, partial pivoting over the columns not yet used); k_gj_update
+// applies it, from one of the two buffers A and inv(A) to the other, so that its tiles read the pivot
+// columns' old values themselves (copied aside by the panel's CTA, an entry per sector, they took half of
+// the panel's time for 912 matrices and a quarter for one).  (Pivots are searched along rows because
 // rows are contiguous, and because the matrices inverted most are eigenvector matrices, whose columns
 // have unit norm: the inverse's error there is 0.86 to 0.94 of the row-pivoted LU's at n = 162 to 338,
 // with column panels 1.2 to 1.3.)
@@ -229,9 +232,9 @@ __global__ void __launch_bounds__(32 * NW) k_inv_reg(int n, const cplx<float>* _
 // eliminated in sub-panels of 8 rows held in registers, a column per thread: a step is one barrier
 // (every warp's best candidate column goes to shared memory with its key, every thread then picks the
 // winner) and 8 complex FMAs per column; the other rows of the panel follow as a rank-8 update.
-// Bound by that chain of barriers (n = 242: ~40 us for one matrix, 170 us for 912, three per SM).
-// With the updates, n = 242: one matrix 1349 -> 406 us, 912 matrices 7.2 -> 4.5 ms against the blocked
-// LU with substitutions on the identity.
+// Bound by that chain of barriers (n = 242: ~30 us for one matrix, two thirds of it the steps).
+// An inverse with its updates, against the blocked LU with substitutions on the identity: one n = 242
+// 1349 -> 318 us, 912 7.2 -> 4.16 ms.
 // ------------------------------------------------------------------------------------------
 constexpr int kGjW = 32;   // panel width
 constexpr int kGjSub = 8;  // sub-panel width
@@ -246,8 +249,7 @@ constexpr size_t gj_panel_smem(int n, int w, int threads) {
 
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT) k_gj_panel(int n, int kb, int w, cplx<T>* A, int64_t lda, int64_t bsA,
-                                                    cplx<T>* U, int64_t ldu, int64_t bsU, int copy_u, int* piv,
-                                                    int* info) {
+                                                    int* piv, int* info) {
   using ct = cplx<T>;
   extern __shared__ __align__(16) unsigned char dyn_gj[];
   __shared__ unsigned ckey[2][32];
@@ -351,62 +353,87 @@ __global__ void __launch_bounds__(MAXT) k_gj_panel(int n, int kb, int w, cplx<T>
     __syncthreads();
   }
   if (tid < w) pv[kb + tid] = pcol[tid];
-  // the pivot columns' old values (rows outside the panel) to U, then the panel back
-  if (r < n) {
-    if (copy_u) {
-      ct* Ub = U + b * bsU;
-#pragma unroll 8
-      for (int c = 0; c < w; ++c) Ub[(int64_t)c * ldu + r] = Ab[(int64_t)r * lda + pcol[c]];
-    }
-    // (a thread of the panel's own rows may have read U's entries before or after these stores: the
-    // update uses none of them)
+  if (r < n)
     for (int c = 0; c < w; ++c) Ab[(int64_t)(kb + c) * lda + r] = P[c * n + r];
-  }
   if (tid == 0 && st) info[b] |= st;
 }
 
-// The update of every row outside the panel [kb, kb + w), in place; or, for the last panel, from
-// A to out with the inverse's rows and columns interchanged (inv[p_r][k] = B[r][p_k]) and the pivot
-// columns read from A itself.  Tiles of 16 TM x 16 TN, TM x TN outputs per thread, the whole rank in one
-// pass through shared memory: 64 x 64 in FP32; 16 x 16 in FP64, whose pipe is so slow (2 FMAs per clock
-// and SM) that padding and idle SMs cost more than the extra loads.  Bound by reading and writing the matrix once per panel and by the issue of
-// the FMAs beside their shared-memory loads: 435 us for 912 matrices of n = 242 (0.86 GB, 2.0 TB/s;
-// 31 TFLOP/s).  128 threads with 8 x 4 outputs each were slower (161 against 139 us for 304: three CTAs
-// of four warps per SM do not cover the loads).
+// The update by the panel of rows [kb, kb + w), from A to out (panel rows copied); for the last panel
+// with the inverse's rows and columns interchanged (inv[p_r][k] = B[r][p_k]).  Tiles of 16 TM x 16 TN,
+// TM x TN outputs per thread, the whole rank in one pass through shared memory: 64 x 64 in FP32; 16 x 16 in
+// FP64, whose pipe is so slow (2 FMAs per clock and SM) that padding and idle SMs cost more than the extra
+// loads.  FP32 products as packed pairs of neighbouring columns (the same FMAs in the same order, half
+// the instructions): 152 matrices of n = 242 895 -> 869 us, 912 4.23 -> 4.16 ms an inverse.  Bound by reading and
+// writing the matrix once per panel (0.86 GB for those 912, 2.4 TB/s with the gathered pivot entries).
+// Slower or no faster: 128 threads with 8 x 4 outputs each (161 against 139 us for 304), a CTA per row of
+// tiles with its pivot entries gathered once (4.21 ms).
 template <typename T, int TM, int TN>
 constexpr size_t gj_update_smem() {
-  return sizeof(cplx<T>) * kGjW * 16 * (TM + TN) + 16 * (TM + TN) * sizeof(int);
+  // (FP32: a pivot column's entry twice, as the packed products take it)
+  return sizeof(cplx<T>) * kGjW * (16 * TN + (16 * TM + 1) * (sizeof(T) == 4 ? 2 : 1)) +
+         16 * (TM + TN) * sizeof(int);
+}
+
+// d = a b + d on two FP32 values each (one instruction for two FMAs, at the FP32 pipe's rate).
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
 }
 
 template <typename T, int TM, int TN>
 __global__ void __launch_bounds__(256, 3) k_gj_update(
-    int n, int kb, int w, cplx<T>* A, int64_t lda, int64_t bsA, const cplx<T>* U, int64_t ldu, int64_t bsU,
-    const int* __restrict__ piv, cplx<T>* out, int64_t ldo, int64_t bsO, int64_t boff) {
+    int n, int kb, int w, const cplx<T>* __restrict__ A, int64_t lda, int64_t bsA, const int* __restrict__ piv,
+    cplx<T>* __restrict__ out, int64_t ldo, int64_t bsO, int last, int64_t boff) {
   using ct = cplx<T>;
   struct alignas(2 * sizeof(ct)) Pair { ct a, b; };
-  constexpr int BM = 16 * TM, BN = 16 * TN;
+  constexpr int BM = 16 * TM, BN = 16 * TN, LU = BM + 1;
   extern __shared__ __align__(32) unsigned char dyn_gu[];
-  ct* Us = reinterpret_cast<ct*>(dyn_gu);  // [w][BM]: the tile's rows of the pivot columns
-  ct* Gs = Us + kGjW * BM;                 // [w][BN]
-  int* col_k = reinterpret_cast<int*>(Gs + kGjW * BN);  // [BN]: step of the column in this panel (or, last, overall)
+  constexpr bool kPacked = sizeof(T) == 4;
+  ct* Gs = reinterpret_cast<ct*>(dyn_gu);  // [w][BN]; packed: real parts [w][BN], then imaginary parts
+  T* Gi = reinterpret_cast<T*>(Gs) + kGjW * BN;
+  // [w][LU]: the tile's rows of the pivot columns; packed: {re, re, im, im}
+  ct* Us = Gs + kGjW * BN;
+  int* col_k = reinterpret_cast<int*>(Us + kGjW * LU * (kPacked ? 2 : 1));  // [BN]: step of the column in this panel (or, last, overall)
   int* row_p = col_k + BN;                              // [BM]: last panel: pivot column of the row's step
   const int64_t b = blockIdx.z + boff;
   const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;  // rows ty + 16 i
   auto col = [&](int j) { return TN == 1 ? tx : 2 * tx + (j & 1) + 32 * (j >> 1); };
-  ct* Ab = A + b * bsA;
+  const ct* Ab = A + b * bsA;
+  ct* Ob = out + b * bsO;
   const int* pv = piv + b * n;
-  const bool last = out != nullptr;
+  {  // a row's pivot columns by neighbouring lanes: they share its lines
+    const int lw = w <= 8 ? 3 : 5, c = tid & ((1 << lw) - 1);
+    if (c < w) {
+      const int p = pv[kb + c];
+#pragma unroll 4
+      for (int i = tid >> lw; i < BM; i += 256 >> lw) {
+        const ct u = row0 + i < n ? Ab[(int64_t)(row0 + i) * lda + p] : mk(T(0));
+        if constexpr (kPacked) reinterpret_cast<float4*>(Us)[c * LU + i] = make_float4(u.re, u.re, u.im, u.im);
+        else Us[c * LU + i] = u;
+      }
+    }
+  }
   if (tid < BN) col_k[tid] = -1;
-  static_assert(BM == BN, "one loop stages both tiles");
-  for (int e = tid; e < w * BM; e += 256) {
-    const int c = e / BM, i = e % BM;
-    ct u = mk(T(0));
-    if (row0 + i < n)
-      u = last ? Ab[(int64_t)(row0 + i) * lda + pv[kb + c]] : U[b * bsU + (int64_t)c * ldu + row0 + i];
-    Us[e] = u;
-    Gs[e] = col0 + i < n ? Ab[(int64_t)(kb + c) * lda + col0 + i] : mk(T(0));
+  for (int e = tid; e < w * BN; e += 256) {
+    const int c = e / BN, i = e % BN;
+    const ct g = col0 + i < n ? Ab[(int64_t)(kb + c) * lda + col0 + i] : mk(T(0));
+    if constexpr (kPacked) {
+      reinterpret_cast<T*>(Gs)[e] = g.re;
+      Gi[e] = g.im;
+    } else {
+      Gs[e] = g;
+    }
   }
   ct acc[TM][TN];
 #pragma unroll
@@ -429,43 +456,84 @@ __global__ void __launch_bounds__(256, 3) k_gj_update(
 #pragma unroll
       for (int i = 0; i < TM; ++i) acc[i][j] = mk(T(0));
     }
-#pragma unroll 4
-  for (int c = 0; c < w; ++c) {
-    ct u[TM], g[TN];
+  if constexpr (kPacked) {
+    using u64 = unsigned long long;
+    u64 re[TM][TN / 2], im[TM][TN / 2];  // of two neighbouring columns
 #pragma unroll
-    for (int i = 0; i < TM; ++i) u[i] = Us[c * BM + ty + 16 * i];
-    if constexpr (TN == 1) {
-      g[0] = Gs[c * BN + tx];
-    } else {
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; j += 2) {
-        const Pair p = *reinterpret_cast<const Pair*>(Gs + c * BN + 2 * tx + 16 * j);
-        g[j] = p.a;
-        g[j + 1] = p.b;
+      for (int j = 0; j < TN / 2; ++j) {
+        re[i][j] = pack2(acc[i][2 * j].re, acc[i][2 * j + 1].re);
+        im[i][j] = pack2(acc[i][2 * j].im, acc[i][2 * j + 1].im);
+      }
+#pragma unroll 2
+    for (int c = 0; c < w; ++c) {
+      u64 gr[TN / 2], gi[TN / 2], ngi[TN / 2];
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) {
+        gr[j] = *reinterpret_cast<const u64*>(reinterpret_cast<const T*>(Gs) + c * BN + 2 * tx + 32 * j);
+        gi[j] = *reinterpret_cast<const u64*>(Gi + c * BN + 2 * tx + 32 * j);
+        ngi[j] = gi[j] ^ 0x8000000080000000ull;
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const ulonglong2 u = reinterpret_cast<const ulonglong2*>(Us)[c * LU + ty + 16 * i];
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) {
+          fma2(re[i][j], u.x, gr[j]);
+          fma2(re[i][j], u.y, ngi[j]);
+          fma2(im[i][j], u.x, gi[j]);
+          fma2(im[i][j], u.y, gr[j]);
+        }
       }
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) fma_acc(acc[i][j], u[i], g[j]);
+      for (int j = 0; j < TN / 2; ++j) {
+        const float2 a = unpack2(re[i][j]), b = unpack2(im[i][j]);
+        acc[i][2 * j] = mk(a.x, b.x);
+        acc[i][2 * j + 1] = mk(a.y, b.y);
+      }
+  } else {
+#pragma unroll 4
+    for (int c = 0; c < w; ++c) {
+      ct u[TM], g[TN];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) u[i] = Us[c * LU + ty + 16 * i];
+      if constexpr (TN == 1) {
+        g[0] = Gs[c * BN + tx];
+      } else {
+#pragma unroll
+        for (int j = 0; j < TN; j += 2) {
+          const Pair p = *reinterpret_cast<const Pair*>(Gs + c * BN + 2 * tx + 16 * j);
+          g[j] = p.a;
+          g[j + 1] = p.b;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma_acc(acc[i][j], u[i], g[j]);
+    }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int rl = ty + 16 * i, r = row0 + rl;
     if (r >= n) continue;
     const bool panel = r >= kb && r < kb + w;
-    if (!last && panel) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int cl = col(j), c = col0 + cl;
       if (c >= n) continue;
-      if (!last) {
-        Ab[(int64_t)r * lda + c] = acc[i][j];
-      } else {
-        ct v = acc[i][j];
-        if (panel) v = Gs[(r - kb) * BN + cl];
-        out[b * bsO + (int64_t)row_p[rl] * ldo + col_k[cl]] = v;
+      ct v = acc[i][j];
+      if (panel) {
+        const int e = (r - kb) * BN + cl;
+        if constexpr (kPacked) v = mk(reinterpret_cast<const T*>(Gs)[e], Gi[e]);
+        else v = Gs[e];
       }
+      if (last) Ob[(int64_t)row_p[rl] * ldo + col_k[cl]] = v;
+      else Ob[(int64_t)r * ldo + c] = v;
     }
   }
 }
@@ -499,19 +567,26 @@ int inverse_panels(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, c
       cudaFuncSetAttribute(update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usmem) != cudaSuccess)
     return KHP_ERR_CUDA;
   const int tiles = (n + 16 * TT - 1) / (16 * TT);
-  for (int kb = 0; kb < n; kb += w) {
-    const int cw = std::min(w, n - kb);
-    const bool last = kb + cw >= n;
-    // the pivot columns' old values wait in the first rows of the output, free until the last panel
-    panel<<<(unsigned)batch, threads, psmem, s>>>(n, kb, cw, A, lda, bsA, Ainv, ldi, bsI, last ? 0 : 1, piv,
-                                                          info);
+  // an odd number of panels, so that the last one goes from A to Ainv: with an even one the first w rows
+  // are taken as two panels
+  const bool odd = (n + w - 1) / w % 2 == 1;
+  cplx<T>* src = A;
+  cplx<T>* dst = Ainv;
+  int64_t lds = lda, bss = bsA, ldd = ldi, bsd = bsI;
+  for (int kb = 0; kb < n;) {
+    const int cw = !odd && kb == 0 ? w / 2 : !odd && kb < w ? w - kb : std::min(w, n - kb);
+    const int last = kb + cw >= n ? 1 : 0;
+    panel<<<(unsigned)batch, threads, psmem, s>>>(n, kb, cw, src, lds, bss, piv, info);
     for (int64_t off = 0; off < batch; off += kMaxGridY) {
       const unsigned nb = (unsigned)std::min<int64_t>(batch - off, kMaxGridY);
-      update<<<dim3(tiles, tiles, nb), 256, usmem, s>>>(n, kb, cw, A, lda, bsA, Ainv, ldi, bsI, piv,
-                                                               last ? Ainv : nullptr, ldi, bsI, off);
+      update<<<dim3(tiles, tiles, nb), 256, usmem, s>>>(n, kb, cw, src, lds, bss, piv, dst, ldd, bsd, last, off);
       count_launches(1);
     }
     count_launches(1);
+    kb += cw;
+    std::swap(src, dst);
+    std::swap(lds, ldd);
+    std::swap(bss, bsd);
   }
   return cuda_status();
 }
