@@ -4,7 +4,7 @@
 // anonymous namespace (uses Elem / MapPtrs / Table and the vector helpers defined there).
 //
 // Notation.  The forward unknowns x (gap amplitudes c+/-, patterned-layer mode amplitudes a+/-,
-// r, t) solve F x = b, F being the interface equations evaluated by k_stack_residual.  For a
+// r, t) solve F x = b, F being the interface equations evaluated by stack_residual.  For a
 // real loss L(r, t) with holomorphic partials g = dL/dx, the adjoint y solves F^T y = g and
 // every parameter theta of F contributes dL = -2 Re(y^T dF/dtheta x).  A patterned layer enters
 // F only through X~ = W diag(exp(-lam k0 d)) W^-1 and Y = V W^-1 (= Q M^-1/2); the gradient with
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(128) k_flux_grad(int nh, int npol, const cd* _
 // RHO = F^T y - g in the layout of the unknowns (X, XA, RT), FP64.  Y in the residual layout.
 // ------------------------------------------------------------------------------------------
 // y_zero: Y is zero (the first round), so are the layers' products.  use_df: the products in double-float
-// on the FP32 pipe (as k_stack_residual; the FP64 pipe's 8 FMAs per element bound them otherwise), with
+// on the FP32 pipe (as stack_residual; the FP64 pipe's 8 FMAs per element bound them otherwise), with
 // their operands as pairs in dfx ([batch][20 n] entries).
 __global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual_T(
     Table tb, const double* gx, const double* gy, const double* kp, const double* k0v, const cd* __restrict__ Y,
@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual_T(
 }
 
 // ------------------------------------------------------------------------------------------
-// Transposed FP32 sweep: Y += Sweep^T RHO, Sweep being the linear map of k_stack_sweep
-// (residual -> correction).  Statements of k_stack_sweep in reverse order, each transposed.
+// Transposed FP32 sweep: Y += Sweep^T RHO, Sweep being the linear map of stack_sweep
+// (residual -> correction).  Statements of stack_sweep in reverse order, each transposed.
 // Per-problem FP32 workspace [..][n][2]: s-bar at every gap (L+1), per layer 4 vectors, 8 temps.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(32 * kPartWarps) k_stack_sweep_T(Table tb, const double* gx, const double* gy,

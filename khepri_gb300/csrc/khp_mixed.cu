@@ -744,14 +744,10 @@ __device__ __forceinline__ cd src_col(const M2* S, int q, int nh, int i, int c) 
 __device__ __forceinline__ cd xprop(const cd* lam64, int i, double dk) { return cexp(-(lam64[i] * dk)); }
 
 // FP64 residual of the stack equations at the current unknowns x (see the Elem comments).
-__global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual(Table tb, const double* gx, const double* gy,
-                                                        const double* kp, const double* k0v, const cd* __restrict__ X,
-                                                        const cd* __restrict__ XA, const cd* __restrict__ RT,
-                                                        cd* RES, cd* scratch, const int* active, int x_zero,
-                                                        int use_df) {
-  TeamCta t;
+__device__ __forceinline__ void stack_residual(const TeamCta& t, const Table& tb, const double* gx, const double* gy,
+                                               const double* kp, const double* k0v, const cd* X, const cd* XA,
+                                               const cd* RT, cd* RES, cd* scratch, bool x_zero, bool use_df) {
   const int64_t b = blockIdx.x;
-  if (active && !active[b]) return;
   if (x_zero) {
     // every unknown is zero (the first round): only the incidence source terms remain, and the
     // FP64 products of the layers would multiply zeros
@@ -878,14 +874,12 @@ __global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual(Table tb, co
 }
 
 // FP32 affine sweep: solves the stack equations for the residual RES (correction system) with
-// the kept factors, and adds the correction to the FP64 unknowns.
+// the kept factors, and adds the correction to the FP64 unknowns.  Returns (to every thread) the largest
+// |correction| of r and t.
 // Per problem workspace (FP32, [..][n][2]): s at every gap (L+1), per layer 5 vectors, 6 temps.
-__global__ void __launch_bounds__(32 * kPartWarps) k_stack_sweep(Table tb, const double* gx, const double* gy, const double* kp,
-                                                     const double* k0v, const cd* __restrict__ RES, cd* X, cd* XA,
-                                                     cd* RT, cf* WS, double* corr, const int* active) {
-  __shared__ TeamShared sh;
-  TeamCta t;
-  if (active && !active[blockIdx.x]) return;
+__device__ __forceinline__ double stack_sweep(const TeamCta& t, const Table& tb, const double* gx, const double* gy,
+                                              const double* kp, const double* k0v, const cd* RES, cd* X, cd* XA, cd* RT,
+                                              cf* WS, TeamShared& sh) {
   double cmax = 0.0;  // largest |correction| of r and t (this thread)
   const int64_t b = blockIdx.x;
   const int nh = tb.nh, n = 2 * nh, L = tb.L;
@@ -1111,27 +1105,38 @@ __global__ void __launch_bounds__(32 * kPartWarps) k_stack_sweep(Table tb, const
   }
   int where = 0;
   team_argmax(t, cmax, where, &sh);
-  if (t.tid() == 0) corr[b] = cmax;
+  return cmax;
 }
 
-// Convergence of the iterative refinement from the last two correction sizes: with linear
-// convergence at rate c1 / c0 the remaining error is about c1^2 / (c0 - c1).  A problem stays
-// active (needs more rounds) while its estimate exceeds 1e-9, its corrections do not shrink,
-// or they are not finite; only problems already active are examined (null: all).
-__global__ void k_check_refine(int64_t batch, const double* __restrict__ c0, const double* __restrict__ c1,
-                               int* active) {
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
-    if (!active[b]) continue;
-    const double a = c0[b], z = c1[b];
-    const bool ok = z == 0.0 || (z < a && z * z <= 1e-9 * (a - z));
-    active[b] = ok ? 0 : 1;
+// The iterative refinement of one problem's stack equations, a CTA per problem: `refine` rounds after the
+// first, in double-float products, then up to kExtraRounds more while the estimated error is above 1e-9 (an
+// ill-conditioned stack next to a Wood anomaly, whose corrections stall at the double-float floor), in
+// FP64.  The estimate is from the last two correction sizes: with linear convergence at rate c1 / c0 the
+// remaining error is about c1^2 / (c0 - c1).  A problem still above it, whose corrections do not shrink or
+// are not finite, gets status bit 8.
+//
+// Problems are independent, so the rounds are one launch: as two or three launches a round, most of
+// them for rounds that no problem took, they were 45 of a call's 190 (one 5 x 5 structure 3.65 -> 3.41 ms a
+// call, 912 problems of n = 242 48 -> 41 ms for all rounds).
+__global__ void __launch_bounds__(32 * kPartWarps) k_stack_refine(
+    const __grid_constant__ Table tb, const double* gx, const double* gy, const double* kp, const double* k0v, cd* X,
+    cd* XA, cd* RT, cd* RES, cd* scratch, cf* WS, int refine, cd epsi, int* status) {
+  __shared__ TeamShared sh;
+  TeamCta t;
+  const int64_t b = blockIdx.x;
+  double c0 = 0.0;
+  bool open = true;
+  const int total = refine >= 1 ? refine + kExtraRounds : 0;
+#pragma unroll 1
+  for (int it = 0; open && it <= total; ++it) {
+    stack_residual(t, tb, gx, gy, kp, k0v, X, XA, RT, RES, scratch, it == 0, it <= refine);
+    t.sync();
+    const double c1 = stack_sweep(t, tb, gx, gy, kp, k0v, RES, X, XA, RT, WS, sh);
+    if (it >= refine) open = !(c1 == 0.0 || (c1 < c0 && c1 * c1 <= 1e-9 * (c0 - c1)));
+    c0 = c1;
+    t.sync();
   }
-}
-
-__global__ void k_flag_unconverged(int64_t batch, const int* __restrict__ active, const double* __restrict__ kp,
-                                   const double* __restrict__ k0, cd epsi, int* status) {
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x)
-    if (active[b] && !rt_undefined(kp + 4 * b, k0[b], epsi)) status[b] |= KHP_BIT_REFINE;
+  if (refine >= 1 && open && t.tid() == 0 && !rt_undefined(kp + 4 * b, k0v[b], epsi)) status[b] |= KHP_BIT_REFINE;
 }
 
 #include "khp_adjoint.cuh"
@@ -1266,8 +1271,6 @@ struct MixedPlan {
   // vectors
   cd *X, *XA, *RT, *RES, *scr;
   cf* SW;
-  double* corr;  // [2][batch]: correction sizes of the last two refinement rounds
-  int* active;   // [batch]: refinement not yet converged
   OzakiWs oz;    // digit arrays of the FP64-accurate tensor-core products (M W and C W)
 };
 
@@ -1363,8 +1366,6 @@ MixedPlan plan_mixed(Arena& a, int64_t batch, int nh, int L, const int* kinds, i
   p.RES = a.take<cd>(batch * (size_t)(L + 2) * 4 * 2 * n);
   p.scr = a.take<cd>(batch * 4 * 2 * n);
   p.SW = a.take<cf>(batch * (size_t)(L + 1 + 5 * L + 6) * 2 * n);
-  p.corr = a.take<double>(2 * (size_t)batch);
-  p.active = a.take<int>(batch);
   return p;
 }
 
@@ -1837,30 +1838,10 @@ int solve_mixed(int64_t batch, int px, int py, int L, const int* kinds, const in
   if (cudaMemsetAsync(p.XA, 0, sizeof(cd) * batch * (size_t)(2 * std::max(L, 1)) * 2 * n, s) != cudaSuccess)
     return KHP_ERR_CUDA;
   if (cudaMemsetAsync(p.RT, 0, sizeof(cd) * batch * 4 * n, s) != cudaSuccess) return KHP_ERR_CUDA;
-  // refine rounds for every problem, then up to kExtraRounds more for the problems whose
-  // estimated error is still above 1e-9 (the others skip them); problems still unconverged get
-  // status bit 8.
-  const int total = refine >= 1 ? refine + kExtraRounds : 0;
-  for (int it = 0; it <= total; ++it) {
-    const int* act = it > refine ? p.active : nullptr;
-    // the refine rounds every problem runs take the products in double-float; the extra rounds
-    // of the problems that have not converged by then (an ill-conditioned stack next to a Wood
-    // anomaly, whose corrections stall at the double-float floor) take them in FP64
-    k_stack_residual<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, gx, gy, kp, k0, p.X, p.XA, p.RT, p.RES, p.scr, act,
-                                                      it == 0 ? 1 : 0, it <= refine ? 1 : 0);
-    count_launches(1);
-    MX_TRY(cuda_status());
-    k_stack_sweep<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, gx, gy, kp, k0, p.RES, p.X, p.XA, p.RT, p.SW,
-                                                   p.corr + (it & 1) * batch, act);
-    count_launches(1);
-    MX_TRY(cuda_status());
-    if (it == refine && refine >= 1) {
-      if (cudaMemsetAsync(p.active, 0xff, sizeof(int) * batch, s) != cudaSuccess) return KHP_ERR_CUDA;
-    }
-    if (it >= refine && refine >= 1)
-      MX_EW(k_check_refine, batch, batch, p.corr + ((it - 1) & 1) * batch, p.corr + (it & 1) * batch, p.active);
-  }
-  if (refine >= 1) MX_EW(k_flag_unconverged, batch, batch, p.active, kp, k0, epsi, status);
+  k_stack_refine<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, gx, gy, kp, k0, p.X, p.XA, p.RT, p.RES, p.scr,
+                                                                  p.SW, refine, epsi, status);
+  count_launches(1);
+  MX_TRY(cuda_status());
   if (!grad) {
     k_flux_cols<double><<<(unsigned)batch, 128, 0, s>>>(nh, npol, p.RT, p.RT + batch * 2 * n, gx, gy, kp, k0,
                                                          reinterpret_cast<const cd*>(te),
