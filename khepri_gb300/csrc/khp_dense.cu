@@ -1027,7 +1027,8 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
     lg = static_cast<unsigned char*>(logbuf);
   // FP32: a warp for the chase, the others for the strips.  While a matrix has an SM to itself more threads
   // than strips shorten their way to and from H (one n = 242: 256 threads 11.2 ms, 288 10.5, 352 9.4, 480
-  // 9.3; n = 162: 4.87, 4.83, 4.09, 4.15; n = 50: 557, 561, 542, 547 us).  Up to two matrices per SM two CTAs
+  // 9.3, 544 with the warps on the chase's scheduler idle 9.0, 480 so 9.2; n = 162: 4.87, 4.83, 4.09, 4.15, 3.94,
+  // 4.21; n = 50: 557, 561, 542, 547, 555, 558 us).  Up to two matrices per SM two CTAs
   // fit with 256 (304 of n = 98: 192 threads 2.67 ms, 256 2.41, 352 3.44).  Beyond, three of 192 where their
   // shared memory fits (456 of n = 98: 192 threads 3.22, 256 4.48; of n = 150: 7.17, 8.87), else two of 288
   // (456 of n = 162: 192 threads 13.8, 256 12.2, 288 11.0; of n = 242: 32.1, 29.5, 25.3).  Small matrices: 512
@@ -1035,7 +1036,7 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   const int sthreads = sizeof(T) == 8 || !lg           ? threads
                        : eig_tuned(n) && batch > 152   ? std::max(64, threads)
                        : n <= 32                       ? 160
-                       : batch <= 152                  ? (n <= 200 ? 352 : 480)
+                       : batch <= 152                  ? (n <= 64 ? 352 : 544)
                        : batch <= 2 * 152              ? kTeamThreads
                        : n <= 150                      ? 192
                                                        : kTeamThreads + 32;

@@ -11,6 +11,7 @@ constexpr int kHqrCols = 32;            // window columns: one per lane
 constexpr int kHqrRot = kHqrCols - 1;   // rotations of a full window
 constexpr int kHqrLd = kHqrCols + 1;    // stride of a window row and of a strip (odd: conflict-free)
 constexpr int kHqrMaxStrips = 640;      // strips staged at a time
+constexpr int kHqrSpareThreads = 512;   // more threads than this leave warp 0's scheduler to it
 
 // Fixed shared memory of cta_hqr (one per CTA); beside it hqr_strips(n) strips of kHqrLd entries.
 // Windows, leading strips and rotations are double-buffered by the window's parity.
@@ -173,13 +174,17 @@ __device__ __forceinline__ void hqr_chase(cplx<T>* win, HqrRot<T>* rot, int nrot
 // with everything else) and by what a window moves between H and shared memory for many (two CTAs per
 // SM).  Against the chase through shared memory with three warp barriers a step and strips from global
 // memory after it (both with the triangular factor's eigenvectors): n = 50 1.35 -> 0.54 ms, n = 98,
-// 64 matrices 3.9 -> 1.74, n = 242 31.0 -> 9.3, 912 matrices 89 -> 43, n = 578 222 -> 72.
+// 64 matrices 3.9 -> 1.72, n = 242 31.0 -> 9.0, 912 matrices 89 -> 43, n = 578 222 -> 72.
 template <typename T>
 __device__ __forceinline__ void cta_hqr_sweep(cplx<T>* H, int64_t ld, int n, int lo, int hi, cplx<T> mu,
                                               HqrShared<T>& sh, cplx<T>* strips, HqrRot<T>* log) {
   static_assert(sizeof(cplx<T>) == 8, "strips are staged in 8-byte copies");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wt = blockDim.x - 32, nw = wt >> 5;  // threads and warps beside warp 0
+  // threads and warps beside warp 0; in the largest CTAs the warps that share its scheduler stay idle
+  const int aw = (blockDim.x >> 5) - 1;
+  const bool spare = blockDim.x > kHqrSpareThreads, idle = spare && warp > 0 && (warp & 3) == 0;
+  const int nw = spare ? aw - aw / 4 : aw, wt = 32 * nw;
+  const int vw = spare ? warp - 1 - warp / 4 : warp - 1, vt = 32 * vw + lane;
   const int cap = hqr_strips(n);
   const int nwin = (hi - lo + kHqrRot - 1) / kHqrRot;
   cplx<T> x = mk(T(0)), y = mk(T(0));  // warp 0: column k - 1 of rows k, k + 1
@@ -194,6 +199,7 @@ __device__ __forceinline__ void cta_hqr_sweep(cplx<T>* H, int64_t ld, int n, int
   }
   for (int w = 0; w <= nwin; ++w) {
     __syncthreads();
+    if (idle) continue;
     if (warp == 0) {
       if (w == nwin) continue;
       cplx<T>* win = sh.win[w & 1];
@@ -220,7 +226,6 @@ __device__ __forceinline__ void cta_hqr_sweep(cplx<T>* H, int64_t ld, int n, int
       }
       continue;
     }
-    const int vt = tid - 32, vw = warp - 1;
     if (w > 0) {
       // window w - 1: roll, write back
       cplx<T>* win = sh.win[(w - 1) & 1];
