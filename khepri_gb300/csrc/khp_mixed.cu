@@ -179,6 +179,47 @@ __device__ void cluster_jacobi(int k, ClusterWarp& w, double big) {
   }
 }
 
+// cluster_jacobi for a block of two, by one thread in registers (the same operations): a warp's FP64
+// instruction takes 16 cycles of the SM for one cluster or for 32, and most clusters are pairs.
+__device__ __forceinline__ void pair_jacobi(cd (&K)[4], cd (&X)[4], double big) {
+  X[0] = X[3] = mk(1.0);
+  X[1] = X[2] = mk(0.0);
+  const double ibig = big > 0.0 ? 1.0 / big : 0.0;
+#pragma unroll 1
+  for (int sweep = 0; sweep < 16; ++sweep) {
+    const cd kab = K[1] * ibig, kba = K[2] * ibig;
+    const cd h = (K[0] - K[3]) * (0.5 * ibig);
+    const cf b32 = mk((float)kab.re, (float)kab.im), c32 = mk((float)kba.re, (float)kba.im);
+    const cf den = pair_den(mk((float)h.re, (float)h.im), b32, c32);
+    if (!(cabs(den) > (float)kDegenerateTol)) break;
+    const cf v12 = cdiv(-b32, den), v21 = cdiv(c32, den);
+    const cf det = mk(1.f) - v12 * v21;
+    if (!(cabs(det) > 1e-3f)) break;
+    const float off = fmaxf(fmaxf(fabsf(b32.re), fabsf(b32.im)), fmaxf(fabsf(c32.re), fabsf(c32.im)));
+    const cd p = mk((double)v12.re, (double)v12.im), q = mk((double)v21.re, (double)v21.im);
+    const cd d64 = mk(1.0) - p * q;
+    const cf i32 = cdiv(mk(1.f), det);
+    cd id = mk((double)i32.re, (double)i32.im);
+#pragma unroll
+    for (int it = 0; it < 2; ++it) id = id * (mk(2.0) - d64 * id);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const cd ca = K[2 * r], cb = K[2 * r + 1], xa = X[2 * r], xb = X[2 * r + 1];
+      K[2 * r] = ca + q * cb;
+      K[2 * r + 1] = cb + p * ca;
+      X[2 * r] = xa + q * xb;
+      X[2 * r + 1] = xb + p * xa;
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const cd ra = K[c], rb = K[2 + c];
+      K[c] = id * (ra - p * rb);
+      K[2 + c] = id * (rb - q * ra);
+    }
+    if (off < 1e-15f) break;
+  }
+}
+
 // Shared memory of k_clusters: a ClusterWarp per warp, then (when it fits) the eigenvalues rounded to
 // FP32 and the label, active and size arrays.
 constexpr int kClusterThreads = 256;
@@ -197,7 +238,8 @@ constexpr size_t cluster_smem(int n) { return kClusterWarps + (size_t)n * (sizeo
 // max|mu|) need FP64 to be decided as it would decide them.  Sweep of 151 symmetric
 // 5 x 5 problems 11.7 -> 9.9 ms, gradients of 32 9 x 9 problems 124 -> 102 ms against one thread per cluster
 // and FP64 distances.  With the rotations in FP32 and the blocks shifted, 96 problems of 9 x 7
-// 3.45 -> 1.49 ms a call, the 32 of 9 x 9 7.9 -> 3.5.
+// 3.45 -> 1.49 ms a call, the 32 of 9 x 9 7.9 -> 3.5.  With a thread per pair and eight columns' loads at
+// a time in the labels 1.22 and 3.3; 32 uneven structures 20.6 -> 12.1, 7 x 5 S-matrices 1.35 -> 0.61.
 __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* __restrict__ mu,
                                                               const cf* __restrict__ E, int* lab, int* pos, int* csz,
                                                               int* memb, cf* xc, cd* mu_out, int in_smem) {
@@ -260,8 +302,29 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
       for (int i = t.tid(); i < n; i += t.size()) {
         if (!act[i]) continue;
         int best = lb[i];
-        for (int j = 0; j < n; ++j)
-          if (act[j] && close(i, j)) best = min(best, lb[j]);
+        if (in_smem && scaled) {  // eight columns' loads at a time (a label read a little early is only older)
+          const float2 mi = mf[i];
+          for (int j0 = 0; j0 < n; j0 += 8) {
+            float2 q[8];
+            int a[8], l[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const int j = min(j0 + u, n - 1);
+              q[u] = mf[j];
+              a[u] = act[j];
+              l[u] = lb[j];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const float dr = q[u].x - mi.x, di = q[u].y - mi.y, d2 = dr * dr + di * di;
+              if (!a[u] || l[u] >= best || d2 > hi2) continue;
+              if (d2 < lo2 || close(i, min(j0 + u, n - 1))) best = l[u];
+            }
+          }
+        } else {
+          for (int j = 0; j < n; ++j)
+            if (act[j] && close(i, j)) best = min(best, lb[j]);
+        }
         if (best < lb[i]) {
           lb[i] = best;
           changed = 1;
@@ -293,12 +356,36 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
     mu_out[b * n + i] = m[i] + mk((double)e.re, (double)e.im);
   }
   t.sync();
-  // one warp per cluster of 2..kClusterMax members (r, k: the same for every lane)
+  // a thread per pair
+  for (int i = t.tid(); i < n; i += t.size()) {
+    const int r = lb[i];
+    if (sz[i] != 2 || r == i) continue;
+    const cd m0 = m[r];
+    const int col[2] = {r, i};
+    cd K[4], X[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const cf v = Eb[(int64_t)col[e >> 1] * n + col[e & 1]];
+      K[e] = mk((double)v.re, (double)v.im) + (e == 3 ? m[i] - m0 : mk(0.0));
+    }
+    pair_jacobi(K, X, big);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int64_t j = b * n + col[q];
+      mu_out[j] = K[3 * q] + m0;
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        memb[j * kClusterMax + p] = col[p];
+        xc[j * kClusterMax + p] = mk((float)X[2 * p + q].re, (float)X[2 * p + q].im);
+      }
+    }
+  }
+  // one warp per cluster of 3..kClusterMax members (r, k: the same for every lane)
   const int lane = t.tid() & 31;
   for (int r = t.tid() >> 5; r < n; r += t.size() >> 5) {
     if (lb[r] != r) continue;
     const int k = sz[r];
-    if (k < 2 || k > kClusterMax) continue;
+    if (k < 3 || k > kClusterMax) continue;
     if (lane == 0) {
       int c = 0;
       for (int j = r; j < n && c < k; ++j)
