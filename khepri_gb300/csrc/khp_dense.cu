@@ -964,24 +964,29 @@ int launch_gemm(int64_t batch, int n, int m, int k, cplx<T> alpha, const cplx<T>
   // FP64: 16 x 16 tiles.  The FP64 pipe (2 FMAs per clock and SM) bounds these whatever the tile, so the
   // smallest tile wastes least on padding and spreads one product over the most SMs (one 50 x 50 product
   // 66 us on the 4 SMs of 32 x 32 tiles, 19 here; 64 products of n = 98 0.80 ms at 64 x 64 tiles, 0.40).
+  // 64 x 64 where they waste at most a tenth and leave four tiles per SM: the rank-32 updates of the
+  // large LU read C and K-slices from memory (n = 4802, four systems: 7.2 s a call at 16 x 16, 4.2 so).
   // FP32: 64 x 64 tiles (4 x 4 outputs per thread) once both output dimensions reach 64; 32 x 128
   // (2 x 8) for outputs of at most 32 rows and at least 128 columns (the block rows of the
   // substitutions); else 32 x 32
-  const bool big = sizeof(T) == 4 && n >= 64 && m >= 64;
+  const int64_t t64 = (int64_t)((n + 63) / 64) * ((m + 63) / 64);
+  const bool big = sizeof(T) == 4 ? n >= 64 && m >= 64
+                                  : t64 * batch >= 4 * 152 && 10 * 64 * 64 * t64 <= 11 * (int64_t)n * m;
   const bool wide = sizeof(T) == 4 && !big && n <= 32 && m >= 128;
-  const int BM = sizeof(T) == 8 ? 16 : big ? 64 : 32, BN = sizeof(T) == 8 ? 16 : big ? 64 : wide ? 128 : 32;
+  const int small = sizeof(T) == 8 ? 16 : 32;
+  const int BM = big ? 64 : small, BN = big ? 64 : wide ? 128 : small;
   for (int64_t off = 0; off < batch; off += kMaxGridY) {
     const unsigned nb = (unsigned)std::min<int64_t>(batch - off, kMaxGridY);
     dim3 grid((m + BN - 1) / BN, (n + BM - 1) / BM, nb);
-    if constexpr (sizeof(T) == 8) {
+    if (big) {
+      k_gemm<T, 64, 64, 8><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
+                                                aidx, bidx, bshift, only);
+    } else if constexpr (sizeof(T) == 8) {
       k_gemm<T, 16, 16, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
                                                  aidx, bidx, bshift, only);
     } else if (wide) {
       k_gemm<T, 32, 128, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
                                                   aidx, bidx, bshift, only);
-    } else if (big) {
-      k_gemm<T, 64, 64, 8><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
-                                                aidx, bidx, bshift, only);
     } else {
       k_gemm<T, 32, 32, 16><<<grid, 256, 0, s>>>(n, m, k, alpha, A, lda, bsA, B, ldb, bsB, beta, C, ldc, bsC, off,
                                                  aidx, bidx, bshift, only);
