@@ -11,8 +11,8 @@ flight).  Synthetic seeded inputs: no dataset is involved.
   timed with CUDA events over exactly K steps (barrier + synchronize on both sides).
 * e2e: the same metric through the public batched API (khepri_gb300.batch.solve_rt) from host
   numpy inputs to host R/T, host<->device copies inside the timed region.
-* roofline: the dominant kernels, the FP32 eigensolver of the modes stage (k_gehrd +
-  k_geev_schur): its algorithmic flops per call (100 n^3 per matrix) / its mean launch duration, timed by CUDA
+* roofline: the dominant kernels, the FP32 eigensolver of the modes stage (k_gehrd_cluster,
+  k_gehrd_q, k_geev_schur, k_hqr_apply_log, k_trevc): its algorithmic flops per call (100 n^3 per matrix) / its mean launch duration, timed by CUDA
   events that libkhp records on its stream around each stage (khp_stage_timing), against the
   FP32 FMA throughput measured in this run (khp_probe_fp32_tflops).  The per-stage times and
   the tensor-core products' fraction of the bf16 peak ride along.
@@ -66,10 +66,11 @@ TC_PAIRS = 36
 TC_FLOPS_PER_MATRIX = TC_PAIRS * 2 * (2 * _up128(N_MAT) * _up64(2 * N_MAT) * _up64(2 * N_MAT)
                                       + 2 * _up128(N_MAT // 2) * _up64(2 * N_MAT) * _up64(N_MAT))
 BF16_PEAK = 1935.4  # TFLOP/s, MEASURED_PEAKS.json bf16_tflops (burst)
-# DRAM bytes per matrix of the FP32 eigensolver (read + write of k_gehrd, k_geev_schur and
-# k_hqr_apply_log) at 912 matrices per launch and 128-thread teams, from one ncu capture of the
-# bench's eigensolver launches (dram__bytes_read.sum + dram__bytes_write.sum, one pass)
-GEEV_TRAFFIC_PER_MATRIX = (70947202816 + 18853817088 + 80481979392 + 95487486208 + 1118951936 + 392237056) / 912
+# DRAM bytes per matrix of the FP32 eigensolver (read + write of k_gehrd_cluster, k_gehrd_q, k_geev_schur,
+# k_hqr_apply_log and k_trevc) at 912 matrices per launch, from one ncu capture of the bench's eigensolver
+# launches (dram__bytes_read.sum + dram__bytes_write.sum, one pass)
+GEEV_TRAFFIC_PER_MATRIX = (432241408 + 796601088 + 427098112 + 381501696 + 3294772224 + 30969671680 + 1117687040
+                           + 392848384 + 254064384 + 376354560) / 912
 
 
 def solve_mixed_flops(n, nmaps, npattern, nhomog):
@@ -92,10 +93,10 @@ def parse():
     ap.add_argument("--steps", type=int, default=5)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--batch", type=int, default=912,
-                    help="problems per call (912 = 6 x 152 SMs: six 128-thread eigensolver CTAs per SM)")
-    ap.add_argument("--eig-threads", type=int, default=128,
+                    help="problems per call (912 = 6 x 152 SMs)")
+    ap.add_argument("--eig-threads", type=int, default=0,
                     help="eigensolver threads per CTA for the sweep's 242 x 242 matrices (khp_tune; 0 = the "
-                         "library default, 256)")
+                         "library's choice by size and batch)")
     ap.add_argument("--mode-digits", type=int, default=0, choices=[0, 6, 8],
                     help="7-bit digits per operand of the eigen-refinement steps' M W products (khp_tune; 0 = "
                          "library default)")
@@ -568,9 +569,8 @@ def run_gpu(args):
                               "config": {"batch": B, "problems_with_status": bad}}), flush=True)
         return
 
-    # roofline of the dominant kernels: the FP32 eigensolver of the modes stage (k_gehrd +
-    # k_geev_schur + k_hqr_apply_log, ~31 % of the step in the launch list), timed live by the
-    # library's stage events
+    # roofline of the dominant kernels: the FP32 eigensolver of the modes stage (~28 % of the step),
+    # timed live by the library's stage events
     scratch = torch.empty(2048 * 1024, dtype=torch.float64, device=dev)
     fp64_peak = lib.khp_probe_fp64_tflops(_capi.ptr(scratch), scratch.numel(), _capi.stream_ptr())
     fp32_peak = lib.khp_probe_fp32_tflops(_capi.ptr(scratch), 2 * scratch.numel(), _capi.stream_ptr())
@@ -582,13 +582,13 @@ def run_gpu(args):
         achieved = eig_flops / (eig_ms / eig_calls * 1e-3) / 1e12
         stages = {k: {"ms_per_call": v[0] / args.steps, "share": round(v[0] / ms, 4)}
                   for k, v in stage_ms.items() if v[1] > 0}
-        roof = {"bound": "fp32", "kernel": "k_gehrd<float> + k_geev_schur<float> + k_hqr_apply_log<float> (eigensolve "
+        roof = {"bound": "fp32", "kernel": "k_gehrd_cluster + k_gehrd_q + k_geev_schur<float> + k_hqr_apply_log<float> + k_trevc<float> (eigensolve "
                          "stage of khp_solve_batched_mixed)",
                 "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp32_peak if fp32_peak > 0 else None,
                 "traffic": GEEV_TRAFFIC_PER_MATRIX * mats if GEEV_TRAFFIC_PER_MATRIX else None,
                 "traffic_source": "DRAM read + write per matrix from one ncu capture at 912 matrices per launch "
-                                  "(128-thread teams), scaled by the matrices of this launch",
+                                  "scaled by the matrices of this launch",
                 "peak_source": "FP32 FMA pipe measured in this run (khp_probe_fp32_tflops); MEASURED_PEAKS.json "
                                "lists only HBM and bf16",
                 "note": "latency-bound (one CTA per matrix; barriers and dependent loads inside each QR "
@@ -690,7 +690,7 @@ def run_gpu(args):
             "vs_baseline": None, "dtype": "c128", "data": "synthetic (seeded)",
             "config": {"workload": "batched sweep 11x11 (n=242), 256x256 multi-disc map, [P,U,P,U,P], 64 f x "
                                    "32x32 k, both polarisations per S-matrix",
-                       "batch": B, "harmonics": "11x11", "eig_threads": args.eig_threads or 256,
+                       "batch": B, "harmonics": "11x11", "eig_threads": args.eig_threads or "library",
                        "recursion_products": ("3xTF32 tensor cores" if (args.tf32_min_n < 0 and N_MAT >= 128)
                                               or 0 < args.tf32_min_n <= N_MAT else "FP32 pipe"),
                        "precision": ("mixed: FP32 O(n^3) work, FP64 eigen-refinement and %d rounds of FP64 "
