@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "khepri_gb300.h"
+#include "khp_clusters.cuh"
 #include "khp_dense.cuh"
 #include "khp_gamma_kernels.cuh"
 #include "khp_launch.h"
@@ -71,15 +72,6 @@ __device__ __forceinline__ cf pair_den(cf h, cf b, cf c) {
   return (h.re * sq.re + h.im * sq.im >= 0.f) ? h + sq : h - sq;
 }
 
-// Eigenvalue clusters of the refinement: the connected components of the graph joining
-// eigenvalues closer than kClusterTol max|mu|.  Inside a cluster a first-order step converges
-// slowly or not at all (its correction E_ij / (mu_j - mu_i) is not small), so every cluster of
-// 2..kClusterMax members takes the exact eigen-decomposition of its block of diag(mu) + E instead.
-// A component larger than kClusterMax (a chain of close eigenvalues) is split again at a third of
-// the distance, up to kClusterLevels times; what is still too large is treated member by member.
-constexpr double kClusterTol = 1e-3;
-constexpr int kClusterMax = 12;
-constexpr int kClusterLevels = 4;
 // Cluster members whose 2x2 sub-block does not resolve two directions (|den| below this times
 // max|mu|) are degenerate to within the refinement's noise (e.g. the two modes of a
 // two-dimensional representation of a symmetric pixmap at normal incidence): any basis of an
@@ -224,7 +216,7 @@ __device__ __forceinline__ void pair_jacobi(cd (&K)[4], cd (&X)[4], double big) 
 // FP32 and the label, active and size arrays.
 constexpr int kClusterThreads = 256;
 constexpr size_t kClusterWarps = sizeof(ClusterWarp) * (kClusterThreads / 32);
-constexpr size_t cluster_smem(int n) { return kClusterWarps + (size_t)n * (sizeof(float2) + 3 * sizeof(int)); }
+constexpr size_t cluster_smem(int n) { return kClusterWarps + (size_t)n * (sizeof(cf) + 3 * sizeof(int)); }
 
 // Clusters of one refinement step (one CTA per problem).  Writes, per column j: lab[j] (the
 // smallest index of its cluster), pos[j] (its rank among the members), csz[j] (the cluster size,
@@ -252,7 +244,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
   const cd* m = mu + b * n;
   const cf* Eb = E + b * nn;
   ClusterWarp* cw = reinterpret_cast<ClusterWarp*>(dyn_cl) + (t.tid() >> 5);
-  float2* mf = reinterpret_cast<float2*>(dyn_cl + kClusterWarps);
+  cf* mf = reinterpret_cast<cf*>(dyn_cl + kClusterWarps);
   // label, size and "still being split" of every column
   int* lb = in_smem ? reinterpret_cast<int*>(mf + n) : lab + b * n;
   int* sz = in_smem ? lb + n : csz + b * n;
@@ -262,88 +254,11 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
   for (int i = t.tid(); i < n; i += t.size()) {
     big = fmax(big, norm2(m[i]));
     lb[i] = i;
-    if (in_smem) mf[i] = make_float2((float)m[i].re, (float)m[i].im);
+    if (in_smem) mf[i] = mk((float)m[i].re, (float)m[i].im);
   }
   team_argmax(t, big, bi, &sh);
   big = sqrt(big);
-  double tol = kClusterTol * big;
-  for (int level = 0; level < kClusterLevels; ++level, tol *= (1.0 / 3.0)) {
-    if (t.tid() == 0) changed = 0;
-    t.sync();
-    for (int i = t.tid(); i < n; i += t.size()) {
-      act[i] = level == 0 || sz[i] > kClusterMax;
-      if (act[i]) {
-        lb[i] = i;
-        changed = 1;
-      }
-    }
-    t.sync();
-    if (!changed) break;
-    t.sync();
-    const double tol2 = tol * tol;
-    const float margin = (float)(1e-6 * big / tol) + 1e-6f;  // (of d2: twice that of d, rounded up)
-    const float lo2 = (1.f - margin) * (float)tol2, hi2 = (1.f + margin) * (float)tol2;
-    const bool scaled = lo2 > 1e-30f && hi2 < 1e30f;  // FP32 squares in range
-    auto close = [&](int i, int j) -> bool {
-      if (in_smem && scaled) {
-        const float dr = mf[j].x - mf[i].x, di = mf[j].y - mf[i].y, d2 = dr * dr + di * di;
-        if (d2 > hi2) return false;
-        if (d2 < lo2) return true;
-      }
-      const double dr = m[j].re - m[i].re, di = m[j].im - m[i].im;
-      return dr * dr + di * di < tol2;
-    };
-    // connected components among the columns being split, by repeated minimum-label propagation
-    // (bounded; a component whose labels have not settled is only split further, and each part is
-    // still handled consistently)
-    for (int it = 0; it < 64; ++it) {
-      if (t.tid() == 0) changed = 0;
-      t.sync();
-      for (int i = t.tid(); i < n; i += t.size()) {
-        if (!act[i]) continue;
-        int best = lb[i];
-        if (in_smem && scaled) {  // eight columns' loads at a time (a label read a little early is only older)
-          const float2 mi = mf[i];
-          for (int j0 = 0; j0 < n; j0 += 8) {
-            float2 q[8];
-            int a[8], l[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int j = min(j0 + u, n - 1);
-              q[u] = mf[j];
-              a[u] = act[j];
-              l[u] = lb[j];
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const float dr = q[u].x - mi.x, di = q[u].y - mi.y, d2 = dr * dr + di * di;
-              if (!a[u] || l[u] >= best || d2 > hi2) continue;
-              if (d2 < lo2 || close(i, min(j0 + u, n - 1))) best = l[u];
-            }
-          }
-        } else {
-          for (int j = 0; j < n; ++j)
-            if (act[j] && close(i, j)) best = min(best, lb[j]);
-        }
-        if (best < lb[i]) {
-          lb[i] = best;
-          changed = 1;
-        }
-      }
-      t.sync();
-      if (!changed) break;
-      t.sync();
-    }
-    // component sizes of the columns just labelled (a label is the smallest index of its
-    // component, so it never equals the label of a column outside it)
-    for (int i = t.tid(); i < n; i += t.size()) {
-      if (!act[i]) continue;
-      int c = 0;
-      for (int j = 0; j < n; ++j) c += lb[j] == lb[i];
-      sz[i] = c;
-    }
-    t.sync();
-  }
+  cluster_labels(t, n, m, in_smem ? mf : nullptr, big, lb, sz, act, &changed);
   // ranks (deterministic: by index)
   for (int i = t.tid(); i < n; i += t.size()) {
     const int l = lb[i];
