@@ -30,6 +30,13 @@ __device__ __forceinline__ unsigned pivot_key(cplx<double> v) {
   if (!(x == x)) return 0u;
   return x == 0.0 ? 1u : max((unsigned)__double2hiint(x), 1u) + 1u;
 }
+// Status of a step from its best candidate's key.  An infinite pivot would eliminate with a reciprocal of
+// 0 and leave a finite "inverse" of a matrix that has none.
+template <typename T>
+__device__ __forceinline__ int pivot_status(unsigned best) {
+  constexpr unsigned kInf = (sizeof(T) == 4 ? 0x7f800000u : 0x7ff00000u) + 1u;
+  return best == 1u ? KHP_BIT_SINGULAR : best == 0u || best >= kInf ? KHP_BIT_NONFINITE : 0;
+}
 
 // 1/p for a pivot (nonzero): conj(p)/|p|^2 with p scaled by a power of two to a modulus of 1 to 2^1.5, one
 // division.  (khp_core.cuh's cdiv takes three divisions in a row and a branch, which every elimination
@@ -111,7 +118,7 @@ __global__ void __launch_bounds__(32 * NW) k_inv_reg(int n, const cplx<float>* _
     pv.re = __shfl_sync(0xffffffffu, pv.re, p & 31);
     pv.im = __shfl_sync(0xffffffffu, pv.im, p & 31);
     const bool ok = best > 1u;  // 1: every candidate is 0; 0: every candidate is NaN
-    if (!ok) st |= best == 1u ? KHP_BIT_SINGULAR : KHP_BIT_NONFINITE;
+    st |= pivot_status<float>(best);
     if (lane == 0) {
       pinv_s[buf] = ok ? pivot_recip(pv) : mk(0.f);
       pcol_s[buf] = ok ? p : ~p;  // ~p: the column is spent but nothing is eliminated
@@ -308,7 +315,7 @@ __global__ void __launch_bounds__(MAXT) k_gj_panel(int n, int kb, int w, cplx<T>
       const unsigned top = __reduce_max_sync(0xffffffffu, kk);
       const int bw = __ffs(__ballot_sync(0xffffffffu, kr >= 0 && kk == top)) - 1;
       const int br = __shfl_sync(0xffffffffu, kr, bw);
-      if (top <= 1u) st |= top == 1u ? KHP_BIT_SINGULAR : KHP_BIT_NONFINITE;
+      st |= pivot_status<T>(top);
       if (tid == 0) pcol[c0 + c] = br;
       const bool pivot = r == br;
       if (pivot) { mine = true; free_col = false; }
