@@ -144,14 +144,13 @@ __global__ void __launch_bounds__(128) k_flux_grad(int nh, int npol, const cd* _
 // ------------------------------------------------------------------------------------------
 // RHO = F^T y - g in the layout of the unknowns (X, XA, RT), FP64.  Y in the residual layout.
 // ------------------------------------------------------------------------------------------
-// y_zero: Y is zero (the first round), so are the layers' products.  use_df: the products in double-float
-// on the FP32 pipe (as stack_residual; the FP64 pipe's 8 FMAs per element bound them otherwise), with
-// their operands as pairs in dfx ([batch][20 n] entries).
+// y_zero: Y is zero (the first round), so are the layers' products.  The products are in FP64 in every
+// round: nothing tests the adjoint's convergence, and next to a Wood anomaly, where a round gains a factor
+// of a few, corrections from double-float residuals would stall at their floor.
 __global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual_T(
     Table tb, const double* gx, const double* gy, const double* kp, const double* k0v, const cd* __restrict__ Y,
-    const cd* __restrict__ GR, const cd* __restrict__ GT, cd* RX, cd* RXA, cd* RRT, cd* scratch, float4* dfx,
-    int y_zero, int use_df) {
-  __shared__ cd part[kPartWarps * 32 * 4];
+    const cd* __restrict__ GR, const cd* __restrict__ GT, cd* RX, cd* RXA, cd* RRT, cd* scratch, int y_zero) {
+  __shared__ cd part[kPartWarps * 32 * 2];
   TeamCta t;
   const int64_t b = blockIdx.x;
   const int nh = tb.nh, n = 2 * nh, L = tb.L;
@@ -218,12 +217,6 @@ __global__ void __launch_bounds__(32 * kPartWarps) k_stack_residual_T(
     if (y_zero) {
       for (int e = t.tid(); e < 8 * n; e += t.size()) p1[e] = mk(0.0);  // p1 .. p4 are one block
       t.sync();
-    } else if (use_df && M.W2) {
-      float4* f = dfx + b * 20 * n;
-      for (int e = t.tid(); e < 8 * n; e += t.size()) f[e] = df_of(y1[e]);  // y1 .. y4 are one block
-      t.sync();
-      team_mvT4_df(t, M.W2 + b * nn, n, f, f + 4 * n, p1, p3, part);
-      team_mvT4_df(t, M.V2 + b * nn, n, f + 2 * n, f + 6 * n, p2, p4, part);
     } else {
       team_mvT2(t, W, n, y1, p1, part);
       team_mvT2(t, V, n, y2, p2, part);

@@ -584,50 +584,7 @@ __device__ void team_mv4_df(const TeamCta& t, const float4* __restrict__ A, int 
   }
 }
 
-// ya = A^T xa and yb = A^T xb, as team_mv4_df; a thread per column, the rows split over groups of warps
-// whose partial sums meet in part (kPartWarps x 128 entries of shared memory).  Ends with a barrier.
-constexpr int kPartWarps = 16;  // warps of the largest team
-__device__ void team_mvT4_df(const TeamCta& t, const float4* __restrict__ A, int n, const float4* xa,
-                             const float4* xb, cd* ya, cd* yb, cd* part) {
-  const int lane = t.tid() & 31, warp = t.tid() >> 5, nw = t.size() >> 5;
-  const int nblk = (n + 31) / 32, rg = max(1, nw / nblk), chunk = (n + rg - 1) / rg;
-  for (int w = warp; w < nblk * rg; w += nw) {
-    const int blk = w % nblk, r = w / nblk, j = blk * 32 + lane;
-    const int i1 = min(n, (r + 1) * chunk);
-    float rh[4], rl[4], ih[4], il[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) rh[c] = rl[c] = ih[c] = il[c] = 0.f;
-    if (j < n)
-#pragma unroll 4
-      for (int i = r * chunk; i < i1; ++i) {
-        const float4 a = A[(int64_t)i * n + j];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float4 u = c < 2 ? xa[2 * i + c] : xb[2 * i + c - 2];
-          df_mac(rh[c], rl[c], a.x, a.z, u.x, u.z);
-          df_mac(rh[c], rl[c], -a.y, -a.w, u.y, u.w);
-          df_mac(ih[c], il[c], a.x, a.z, u.y, u.w);
-          df_mac(ih[c], il[c], a.y, a.w, u.x, u.z);
-        }
-      }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const cd v = mk((double)rh[c] + (double)rl[c], (double)ih[c] + (double)il[c]);
-      if (rg > 1) part[(w * 32 + lane) * 4 + c] = v;
-      else if (j < n) (c < 2 ? ya : yb)[2 * j + (c & 1)] = v;
-    }
-  }
-  t.sync();
-  if (rg > 1) {
-    for (int e = t.tid(); e < 4 * n; e += t.size()) {
-      const int j = e >> 2, c = e & 3;
-      cd v = mk(0.0);
-      for (int r = 0; r < rg; ++r) v += part[(r * nblk * 32 + j) * 4 + c];
-      (c < 2 ? ya : yb)[2 * j + (c & 1)] = v;
-    }
-    t.sync();
-  }
-}
+constexpr int kPartWarps = 16;  // warps of the largest team of the stack kernels
 
 __global__ void k_round(int64_t count, const cd* __restrict__ in, cf* out) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x)
@@ -1575,10 +1532,8 @@ int grad_mixed(const Table& tb, MixedPlan& p, GradPlan& g, const GradArgs& ga, i
   if (cudaMemsetAsync(g.Y, 0, sizeof(cd) * batch * (size_t)(L + 2) * 4 * 2 * n, s) != cudaSuccess)
     return KHP_ERR_CUDA;
   for (int it = 0; it < refine + 3; ++it) {
-    // (the products in double-float but for the last round, whose residual decides the accuracy)
     k_stack_residual_T<<<(unsigned)batch, stack_threads(batch), 0, s>>>(
-        tb, gx, gy, kp, k0, g.Y, g.GR, g.GT, g.RX, g.RXA, g.RRT, g.scr4, reinterpret_cast<float4*>(g.VEC), it == 0,
-        it < refine + 2);
+        tb, gx, gy, kp, k0, g.Y, g.GR, g.GT, g.RX, g.RXA, g.RRT, g.scr4, it == 0 ? 1 : 0);
     count_launches(1);
     MX_TRY(cuda_status());
     k_stack_sweep_T<<<(unsigned)batch, stack_threads(batch), 0, s>>>(tb, gx, gy, kp, k0, g.RX, g.RXA, g.RRT, g.Y, g.SWT);
