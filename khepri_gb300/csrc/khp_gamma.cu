@@ -57,7 +57,7 @@ struct GammaPlan {
   // modes scratch (reused per map)
   cplx<T> *M, *Z, *CW, *lu;
   int* piv;
-  char* eig;               // scratch of launch_geev_refined
+  char* eig;               // scratch of launch_geev_refined, over the arrays from Z to P
   size_t eig_bytes;
   std::vector<int*> midx;  // per distinct map: the map index of every problem
   // per layer
@@ -70,7 +70,8 @@ struct GammaPlan {
 };
 
 template <typename T>
-GammaPlan<T> plan_gamma(Arena& a, int64_t batch, int nh, int nlayers, const int* kinds, int nmaps_used) {
+GammaPlan<T> plan_gamma(Arena& a, int64_t batch, int nh, int nlayers, const int* kinds, int nmaps_used,
+                        bool eigensolve) {
   const size_t n = 2 * (size_t)nh, nn = n * n;
   GammaPlan<T> p;
   for (int m = 0; m < nmaps_used; ++m) {
@@ -83,29 +84,28 @@ GammaPlan<T> plan_gamma(Arena& a, int64_t batch, int nh, int nlayers, const int*
     p.midx.push_back(a.take<int>(batch));
   }
   p.M = a.take<cplx<T>>(batch * nn);
+  for (int l = 0; l < nlayers; ++l) p.blocks.push_back(kinds[l] == 1 ? nullptr : a.take<M2>(batch * nh * 4));
+  p.inc = a.take<M2>(batch * nh * 4);
+  p.trn = a.take<M2>(batch * nh * 4);
+  // what the eigensolver may use: nothing of it is written before a map's eigenpairs are there, or read
+  // after the next map's are begun
+  const size_t eig = a.off;
   p.Z = a.take<cplx<T>>(batch * nn);
   p.CW = a.take<cplx<T>>(batch * nn);
   p.lu = a.take<cplx<T>>(batch * nn);
-  p.eig_bytes = nmaps_used > 0 ? geev_refined_workspace(batch, (int)n) : 0;
-  p.eig = a.take<char>(p.eig_bytes);
   p.piv = a.take<int>(batch * n);
   for (int l = 0; l < nlayers; ++l) {
-    if (kinds[l] == 1) {
-      p.inv1.push_back(a.take<cplx<T>>(batch * nn));
-      p.inv2.push_back(a.take<cplx<T>>(batch * nn));
-      p.blocks.push_back(nullptr);
-    } else {
-      p.inv1.push_back(a.take<cplx<T>>(batch * nn));
-      p.inv2.push_back(nullptr);
-      p.blocks.push_back(a.take<M2>(batch * nh * 4));
-    }
+    p.inv1.push_back(a.take<cplx<T>>(batch * nn));
+    p.inv2.push_back(kinds[l] == 1 ? a.take<cplx<T>>(batch * nn) : nullptr);
   }
-  p.inc = a.take<M2>(batch * nh * 4);
-  p.trn = a.take<M2>(batch * nh * 4);
   p.G = a.take<cplx<T>>(batch * nn);
   p.F = a.take<cplx<T>>(batch * nn);
   p.Gb = a.take<cplx<T>>(batch * nn);
   p.P = a.take<cplx<T>>(batch * nn);
+  const size_t span = a.off - eig;
+  p.eig_bytes = eigensolve && nmaps_used > 0 ? geev_refined_workspace(batch, (int)n, span) : 0;
+  if (p.eig_bytes > span) a.take<char>(p.eig_bytes - span);
+  p.eig = a.base ? a.base + eig : nullptr;
   p.u = a.take<cplx<T>>(batch * n * 2);
   p.tmp = a.take<cplx<T>>(batch * n * 2);
   p.rv = a.take<cplx<T>>(batch * n * 2);
@@ -181,7 +181,7 @@ int solve_gamma(int64_t batch, int px, int py, int nlayers, const int* kinds, co
   }
   auto depth_of = [&](int l) { return DepthSel{pdepth ? pdepth + (int64_t)l * batch : nullptr, depths[l]}; };
   Arena a{static_cast<char*>(workspace), ws_bytes};
-  GammaPlan<T> p = plan_gamma<T>(a, batch, nh, nlayers, kinds, (int)used.size());
+  GammaPlan<T> p = plan_gamma<T>(a, batch, nh, nlayers, kinds, (int)used.size(), !given);
   if (!a.ok || !workspace) return KHP_ERR_WORKSPACE;
   const cplx<T> one = mk(T(1)), zero = mk(T(0)), mone = mk(T(-1));
 
@@ -297,7 +297,7 @@ size_t khp_solve_batched_workspace(int64_t batch, int32_t nh, int32_t nlayers, c
   }
   used = (int)seen.size();
   Arena a{nullptr, 0};
-  plan_gamma<double>(a, batch, nh, nlayers, layer_kind, used);
+  plan_gamma<double>(a, batch, nh, nlayers, layer_kind, used, true);
   return a.off;
 }
 

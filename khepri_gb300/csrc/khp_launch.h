@@ -47,8 +47,10 @@ int launch_normalize_cols(int64_t batch, int n, const cplx<T>* V, int64_t ldv, i
                           int64_t bsW, cudaStream_t s, const int* only = nullptr);
 
 // M W = W diag(lam) in FP64 (M [batch][n][n] destroyed; unit columns): FP32 eigensolver and FP64
-// refinement, the matrices whose residual test fails by the FP64 eigensolver (khp_mixed.cu).
-size_t geev_refined_workspace(int64_t batch, int n);
+// refinement, the matrices whose residual test fails by the FP64 eigensolver (khp_mixed.cu).  Scratch: `have`
+// bytes that the caller has free during the call anyway, or more where that lets all matrices go
+// together and comes to at most kRefinedScratch (fewer at a time otherwise).
+size_t geev_refined_workspace(int64_t batch, int n, size_t have);
 int launch_geev_refined(int64_t batch, int n, cplx<double>* M, cplx<double>* W, cplx<double>* lam, int* info,
                         cudaStream_t s, void* ws, size_t ws_bytes);
 

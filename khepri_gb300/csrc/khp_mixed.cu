@@ -1459,18 +1459,17 @@ int refine_eigs(int64_t bm, int n, const cd* M64, cd* W64, EigRefine& r, int ste
 // Workspace of launch_geev_refined.
 struct RefinedWs {
   EigRefine er;
-  cf* M32;   // with Z32 one block: Z of the FP64 eigensolver
+  cf* M32;  // (also F)
   cf* lam32;
-  int *st, *act;
+  int* st;
 };
 
 RefinedWs plan_refined(Arena& a, int64_t batch, int n) {
   const size_t nn = (size_t)n * n, b = (size_t)batch;
   RefinedWs w;
   EigRefine& r = w.er;
-  w.M32 = a.take<cf>(2 * b * nn);
-  r.F32 = w.M32;
-  r.Z32 = w.M32 ? w.M32 + b * nn : nullptr;
+  w.M32 = r.F32 = a.take<cf>(b * nn);
+  r.Z32 = a.take<cf>(b * nn);
   r.W32 = a.take<cf>(b * nn);
   r.Wi = a.take<cf>(b * nn);
   r.E32 = a.take<cf>(b * nn);
@@ -1487,9 +1486,8 @@ RefinedWs plan_refined(Arena& a, int64_t batch, int n) {
   r.xc = a.take<cf>(b * n * kClusterMax);
   r.piv = a.take<int>(b * n);
   w.st = a.take<int>(b);
-  w.act = a.take<int>(b);
   r.st = w.st;
-  const size_t ch = (size_t)ozaki_chunk((int64_t)b);
+  const size_t ch = std::min(b, (size_t)kOzakiMaxChunk);
   r.oz.ad_elems = ch * ozaki_a_elems(n, n);
   r.oz.ad = a.take<uint16_t>(r.oz.ad_elems);
   r.oz.ea_n = ch * ozaki_rows_padded(n);
@@ -1828,44 +1826,81 @@ constexpr int kRefinedMaxN = 4096;  // the digit products' limit
 constexpr double kRefinedTolPerN = 4e-16;
 constexpr int kRefinedSteps = 4;
 
-size_t geev_refined_workspace(int64_t batch, int n) {
+// Scratch: one int per matrix, then the refinement's for as many matrices at a time as there is room for;
+// after it the FP64 eigensolver's Z for all of them.  One n = 242 matrix takes 11.7 MB (Z 0.9 MB), so that
+// 183 of them, a matrix and more per SM, go together within kRefinedScratch; what a larger call has of its
+// own (FP64 recursions 100 to 240 bytes per entry, khp_layer_modes 32) holds at least a sixth of its
+// matrices at a time.  With room for all of them khp_layer_modes took 2.9 to 6.6 times its former workspace.
+constexpr size_t kRefinedScratch = size_t(2) << 30;
+
+namespace {
+size_t refined_mask_bytes(int64_t batch) { return ((size_t)batch * sizeof(int) + 255) & ~size_t(255); }
+size_t refined_bytes(int64_t batch, int n) {
   Arena a{nullptr, 0};
-  if (n < kRefinedMinN || n > kRefinedMaxN) {
-    a.take<cd>((size_t)batch * n * n);  // Z
-  } else {
-    plan_refined(a, batch, n);
-  }
+  plan_refined(a, batch, n);
   return a.off;
+}
+// Matrices at a time within `bytes`, at least one; the slices of a batch are made equal.
+int64_t refined_slice(int64_t batch, int n, size_t bytes) {
+  int64_t lo = 1, hi = batch;
+  while (lo < hi) {
+    const int64_t m = (lo + hi + 1) / 2;
+    if (refined_bytes(m, n) <= bytes) lo = m;
+    else hi = m - 1;
+  }
+  const int64_t parts = (batch + lo - 1) / lo;
+  return (batch + parts - 1) / parts;
+}
+}  // namespace
+
+size_t geev_refined_workspace(int64_t batch, int n, size_t have) {
+  if (batch <= 0) return have;
+  const size_t z = sizeof(cd) * (size_t)batch * n * n;
+  if (n < kRefinedMinN || n > kRefinedMaxN) return std::max(have, z);
+  const size_t mask = refined_mask_bytes(batch);
+  const size_t room = std::max(have, kRefinedScratch);
+  const int64_t slice = refined_slice(batch, n, room > mask ? room - mask : 0);
+  return std::max(have, mask + std::max(z, refined_bytes(slice, n)));
 }
 
 int launch_geev_refined(int64_t batch, int n, cd* M, cd* W, cd* lam, int* info, cudaStream_t s, void* ws,
                         size_t ws_bytes) {
   if (batch <= 0) return KHP_OK;
   const int64_t nn = (int64_t)n * n;
-  Arena a{static_cast<char*>(ws), ws_bytes};
-  if (n < kRefinedMinN || n > kRefinedMaxN) {
-    cd* Z = a.take<cd>((size_t)batch * nn);
-    if (!a.ok || !ws) return KHP_ERR_WORKSPACE;
-    return launch_geev<double>(batch, n, M, n, nn, Z, W, n, nn, lam, n, info, s);
+  const size_t z = sizeof(cd) * (size_t)batch * nn;
+  const bool refined = n >= kRefinedMinN && n <= kRefinedMaxN;
+  const size_t mask = refined ? refined_mask_bytes(batch) : 0;
+  if (!ws || ws_bytes < mask + z) return KHP_ERR_WORKSPACE;
+  char* base = static_cast<char*>(ws) + mask;
+  if (!refined)
+    return launch_geev<double>(batch, n, M, n, nn, reinterpret_cast<cd*>(base), W, n, nn, lam, n, info, s);
+  // act[b]: matrix b is solved in FP64 after all: an FP32 stage failed, or a column's residual is too large
+  int* act = static_cast<int*>(ws);
+  if (cudaMemsetAsync(act, 0, sizeof(int) * batch, s) != cudaSuccess) return KHP_ERR_CUDA;
+  const int64_t slice = refined_slice(batch, n, ws_bytes - mask);
+  for (int64_t o = 0; o < batch; o += slice) {
+    const int64_t bm = std::min(slice, batch - o);
+    Arena a{base, ws_bytes - mask};
+    RefinedWs w = plan_refined(a, bm, n);
+    if (!a.ok) return KHP_ERR_WORKSPACE;
+    EigRefine& r = w.er;
+    cd* Mo = M + o * nn;
+    cd* Wo = W + o * nn;
+    if (cudaMemsetAsync(w.st, 0, sizeof(int) * bm, s) != cudaSuccess) return KHP_ERR_CUDA;
+    MX_EW(k_round, bm * nn, bm * nn, Mo, w.M32);
+    MX_TRY(launch_geev<float>(bm, n, w.M32, n, nn, r.Z32, r.W32, n, nn, w.lam32, n, w.st, s, r.MW64,
+                              (int64_t)(nn * sizeof(cd)) / 32 * 32));
+    MX_TRY(refine_eigs(bm, n, Mo, Wo, r, kRefinedSteps, s));
+    MX_TRY(ozaki_zgemm(bm, n, n, n, Mo, n, nn, nullptr, Wo, n, nn, r.MW64, n, nn, r.oz, s));
+    if (cudaMemcpyAsync(act + o, w.st, sizeof(int) * bm, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+      return KHP_ERR_CUDA;
+    MX_TRY(launch_eig_check(bm, n, r.MW64, Wo, r.mu, nullptr, nullptr, mk(0.0), kRefinedTolPerN * n, 1, act + o, s));
+    if (cudaMemcpyAsync(lam + o * n, r.mu, sizeof(cd) * bm * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+      return KHP_ERR_CUDA;
   }
-  RefinedWs w = plan_refined(a, batch, n);
-  if (!a.ok || !ws) return KHP_ERR_WORKSPACE;
-  EigRefine& r = w.er;
-  if (cudaMemsetAsync(w.st, 0, sizeof(int) * batch, s) != cudaSuccess) return KHP_ERR_CUDA;
-  MX_EW(k_round, batch * nn, batch * nn, M, w.M32);
-  MX_TRY(launch_geev<float>(batch, n, w.M32, n, nn, r.Z32, r.W32, n, nn, w.lam32, n, w.st, s, r.MW64,
-                            (int64_t)(nn * sizeof(cd)) / 32 * 32));
-  MX_TRY(refine_eigs(batch, n, M, W, r, kRefinedSteps, s));
-  MX_TRY(ozaki_zgemm(batch, n, n, n, M, n, nn, nullptr, W, n, nn, r.MW64, n, nn, r.oz, s));
-  // matrices to solve in FP64 after all: an FP32 stage failed, or a column's residual is too large
-  if (cudaMemcpyAsync(w.act, w.st, sizeof(int) * batch, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-    return KHP_ERR_CUDA;
-  MX_TRY(launch_eig_check(batch, n, r.MW64, W, r.mu, nullptr, nullptr, mk(0.0), kRefinedTolPerN * n, 1, w.act, s));
-  if (cudaMemcpyAsync(lam, r.mu, sizeof(cd) * batch * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-    return KHP_ERR_CUDA;
   MX_TRY(launch_normalize_cols<double>(batch, n, W, n, nn, W, n, nn, s));
-  return launch_geev<double>(batch, n, M, n, nn, reinterpret_cast<cd*>(w.M32), W, n, nn, lam, n, info, s, nullptr, 0,
-                             w.act);
+  return launch_geev<double>(batch, n, M, n, nn, reinterpret_cast<cd*>(base), W, n, nn, lam, n, info, s, nullptr, 0,
+                             act);
 }
 
 int mixed_modes_in_workspace(int64_t batch, int nh, int L, const int* kinds, const int* maps, const void* ws,

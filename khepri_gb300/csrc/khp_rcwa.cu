@@ -625,10 +625,14 @@ inline ModesWs plan_modes(Arena& a, int64_t batch, int nh) {
   const size_t n = 2 * (size_t)nh;
   ModesWs w;
   w.M = a.take<cd>(batch * n * n);
-  w.eig_bytes = geev_refined_workspace(batch, (int)n);
-  w.eig = a.take<char>(w.eig_bytes);
+  // the eigensolver's scratch, CW (written after it) among it
+  const size_t eig = a.off;
   w.CWt = a.take<cd>(batch * nh * n);
   w.CWb = a.take<cd>(batch * nh * n);
+  const size_t span = a.off - eig;
+  w.eig_bytes = geev_refined_workspace(batch, (int)n, span + sizeof(cd) * batch * n * n);
+  if (w.eig_bytes > span) a.take<char>(w.eig_bytes - span);
+  w.eig = a.base ? a.base + eig : nullptr;
   return w;
 }
 
