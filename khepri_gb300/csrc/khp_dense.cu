@@ -91,7 +91,7 @@ size_t schur_smem(int n, bool log) {
 // the back-transform W = Z X runs afterwards as a batched tiled product.  With a log
 // region (log_bytes per matrix at logbuf) Z's updates are logged and left for k_hqr_apply_log.
 template <typename T, int MAXT>
-__global__ void __launch_bounds__(MAXT, sizeof(T) == 4 && MAXT < 512 ? 2 : 1) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
+__global__ void __launch_bounds__(MAXT, MAXT < 512 ? 2 : 1) k_geev_schur(int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z,
                                                               cplx<T>* lam, int64_t bsLam, int* info,
                                                               unsigned char* logbuf, int64_t log_bytes,
                                                               const int* __restrict__ only, int vectors) {
@@ -1045,7 +1045,11 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
                        : batch <= 2 * 152              ? kTeamThreads
                        : n <= 150                      ? 192
                                                        : kTeamThreads + 32;
-  auto schur = sthreads <= kTeamThreads + 32 ? k_geev_schur<T, kTeamThreads + 32> : k_geev_schur<T, 2 * kTeamThreads + 32>;
+  // (FP64 teams end at 256, so that two share an SM: with the registers that 288 threads may take only one
+  // fits, and 304 scattering eigenproblems of N = 100 took 154 instead of 94 ms, of N = 36 22 instead of 13)
+  auto schur = k_geev_schur<T, sizeof(T) == 8 ? kTeamThreads : kTeamThreads + 32>;
+  if constexpr (sizeof(T) == 4)
+    if (sthreads > kTeamThreads + 32) schur = k_geev_schur<T, 2 * kTeamThreads + 32>;
   const size_t ssm = schur_smem<T>(n, lg != nullptr);
   if (ssm > 40 * 1024 &&
       cudaFuncSetAttribute(schur, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
