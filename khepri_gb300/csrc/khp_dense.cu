@@ -230,6 +230,8 @@ __global__ void __launch_bounds__(32 * kTrevcWarps) k_trevc(int n, const cplx<T>
 constexpr int kLogRows = 32;
 constexpr int kLogChunk = 256;
 constexpr int kLogAhead = 8;
+// FP64: from this size on; below, the kernel's own 0.1 ms is more than Z's share of the QR.
+constexpr int kLogMinN64 = 33;
 
 template <typename T>
 size_t apply_log_smem(int n) {
@@ -266,12 +268,14 @@ __device__ __forceinline__ void roll_logged(cplx<T>* p, const HqrRot<T>* g, cplx
 
 template <typename T>
 __global__ void __launch_bounds__(kLogRows) k_hqr_apply_log(int n, cplx<T>* Z, const unsigned char* logbuf,
-                                                             int64_t log_bytes, int64_t boff) {
+                                                             int64_t log_bytes, int64_t boff,
+                                                             const int* __restrict__ only) {
   extern __shared__ __align__(32) unsigned char dyn[];
   HqrRot<T>* stage = reinterpret_cast<HqrRot<T>*>(dyn);  // [2][kLogChunk]
   cplx<T>* rows = reinterpret_cast<cplx<T>*>(dyn + 2 * kLogChunk * sizeof(HqrRot<T>));
   const int lds = n | 1;
   const int64_t b = blockIdx.y + boff;
+  if (only && !only[b]) return;
   const HqrLog<T> L = hqr_log_view<T>(const_cast<unsigned char*>(logbuf) + b * log_bytes, log_bytes, n);
   const int nsw = L.head[0], nrot = L.head[1];
   if (nsw <= 0) return;
@@ -1009,7 +1013,12 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(k_gehrd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return KHP_ERR_CUDA;
-  const int threads = eig_threads(n);
+  // (FP64: smaller teams for small matrices, whose barriers and reductions are most of a step; one n = 18
+  // 1.64 ms with 256 threads, 1.55 with 64; n = 50 8.96, 8.76 with 128; n = 98 the fastest with 256)
+  const int threads = sizeof(T) == 8 && !eig_tuned(n) ? (n <= 32   ? 64
+                                                         : n <= 64 ? 128
+                                                                   : kTeamThreads)
+                                                      : eig_threads(n);
   // the blocked reduction keeps full 256-thread teams (its panel updates are parallel work; three
   // teams per SM already cover the SM), whatever team size suits the QR's serial window chase
   const int gthreads = blocked ? kTeamThreads : threads;
@@ -1027,7 +1036,8 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   }
   // Z through the rotation log when the region holds at least one full sweep per matrix
   unsigned char* lg = nullptr;
-  if (logbuf && !only && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
+  const bool log_fits = sizeof(T) == 4 || (n >= kLogMinN64 && apply_log_smem<T>(n) <= 226 * 1024);
+  if (logbuf && log_fits && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
       hqr_log_view<T>(logbuf, log_bytes, n).cap_rot >= n - 1)
     lg = static_cast<unsigned char*>(logbuf);
   // FP32: a warp for the chase, the others for the strips.  While a matrix has an SM to itself more threads
@@ -1069,7 +1079,7 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
       return KHP_ERR_CUDA;
     for (int64_t off = 0; off < batch; off += kMaxGridY) {
       const unsigned nb = (unsigned)std::min<int64_t>(batch - off, kMaxGridY);
-      k_hqr_apply_log<T><<<dim3((n + kLogRows - 1) / kLogRows, nb), kLogRows, lsm, s>>>(n, Z, lg, log_bytes, off);
+      k_hqr_apply_log<T><<<dim3((n + kLogRows - 1) / kLogRows, nb), kLogRows, lsm, s>>>(n, Z, lg, log_bytes, off, only);
       count_launches(1);
     }
     st = cuda_status();

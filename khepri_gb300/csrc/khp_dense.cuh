@@ -515,7 +515,7 @@ KHP_HD cplx<T> hqr_shift(const cplx<T>* H, int64_t ld, int lo, int hi, int its) 
 
 // Givens rotation G = [[c, s], [-conj(s), c]] (c real) with G [x; y] = [r; 0].
 template <typename T>
-KHP_HD void givens(cplx<T> x, cplx<T> y, T& c, cplx<T>& s, cplx<T>& r) {
+KHP_HD void givens_scaled(cplx<T> x, cplx<T> y, T& c, cplx<T>& s, cplx<T>& r) {
   const T ax = cabs(x), ay = cabs(y);
   if (ay == T(0)) { c = T(1); s = mk(T(0)); r = x; return; }
   if (ax == T(0)) { c = T(0); s = conj(y) * (T(1) / ay); r = mk(ay); return; }
@@ -524,6 +524,35 @@ KHP_HD void givens(cplx<T> x, cplx<T> y, T& c, cplx<T>& s, cplx<T>& r) {
   c = ax / rho;
   s = ph * conj(y) * (T(1) / rho);
   r = ph * rho;
+}
+
+// 1 / sqrt(v).
+KHP_HD double khp_rsqrt(double v) {
+#ifdef __CUDA_ARCH__
+  return rsqrt(v);
+#else
+  return 1.0 / std::sqrt(v);
+#endif
+}
+
+template <typename T>
+KHP_HD void givens(cplx<T> x, cplx<T> y, T& c, cplx<T>& s, cplx<T>& r);
+
+// FP64 form with one reciprocal square root, q = 1 / (|x| rho), which scales c and s alike (unitary to its
+// rounding): ~30 operations on the serial chain of the QR sweep, of a pipe that a warp's instruction
+// holds for 16 cycles, where three hypots and three divisions take ~170.  Magnitudes whose fourth powers
+// leave the range take the scaled form.
+template <>
+KHP_HD void givens<double>(cplx<double> x, cplx<double> y, double& c, cplx<double>& s, cplx<double>& r) {
+  const double ax2 = norm2(x), t2 = ax2 + norm2(y);
+  if (!(ax2 >= 1e-140 && t2 <= 1e140)) {
+    givens_scaled(x, y, c, s, r);
+    return;
+  }
+  const double q = khp_rsqrt(ax2 * t2);
+  c = ax2 * q;
+  s = mul_conj(x, y) * q;
+  r = x * (t2 * q);
 }
 
 // FP32 form with reciprocal square roots instead of hypot and divisions (the rotation sits on

@@ -102,6 +102,9 @@ struct OzakiWs {
   int* eb = nullptr;   // B column exponents
   size_t eb_n = 0;
   int* err = nullptr;  // one int: set when a tensor-core tile timed out (the tcgen05 path)
+  // optional, device int[batch] (the tcgen05 path; the other computes all): problems with only[b] == 0 are
+  // left alone
+  const int* only = nullptr;
 };
 constexpr int64_t kOzakiMaxChunk = 256;  // problems per chunk (digit arrays: ~5.5 MB per 242 x 242 problem)
 size_t ozaki_a_elems(int m, int k);  // per problem

@@ -53,9 +53,10 @@ constexpr int kMaxRefine = 64;
 // R32 = (M64 W64 - W64 diag(mu)) in FP32, where MW already holds M64 W64.
 // One grid row per problem (b = boff + blockIdx.y), launched by MX_PP.
 __global__ void k_eig_residual(int64_t boff, int n, const cd* __restrict__ MW, const cd* __restrict__ W64,
-                               const cd* __restrict__ mu, cf* R32) {
+                               const cd* __restrict__ mu, cf* R32, const int* __restrict__ keep) {
   const int64_t nn = (int64_t)n * n;
   const int64_t b = boff + blockIdx.y;
+  if (keep && !keep[b]) return;
   for (int rc = blockIdx.x * blockDim.x + threadIdx.x; rc < nn; rc += gridDim.x * blockDim.x) {
     const int64_t e = b * nn + rc;
     const int j = rc % n;
@@ -77,6 +78,17 @@ __device__ __forceinline__ cf pair_den(cf h, cf b, cf c) {
 // two-dimensional representation of a symmetric pixmap at normal incidence): any basis of an
 // exactly degenerate subspace is an eigenbasis, and a rotation computed from noise is O(1).
 constexpr double kDegenerateTol = 1e-9;
+
+// A matrix is given up by the FP64 refinement (launch_geev_refined) when, before its first step, an eigenvalue
+// has kUnresolved others within kUnresolvedTol max|mu| whose coupling E exceeds kCoupledTol max|mu|: the FP32
+// solver has not separated them, the block of diag(mu) + E is nothing like diagonal, and no step
+// resolves it.  These are weakly modulated maps at normal incidence (contrast 1e-9 to 0.03 and more), by
+// their groups of 8 and 16 harmonics; symmetric structures have pairs, and an unmodulated map couples
+// nothing.  Over 840 matrices of n = 18 to 98 and contrasts 0 to 11 (a model of the steps in numpy): of 435
+// that miss the residual test after all steps 400 are given up here, of 405 that pass 31.
+constexpr int kUnresolved = 5;
+constexpr double kUnresolvedTol = 1e-5;
+constexpr float kCoupledTol = 1e-13f;
 
 // Scratch of one warp's cluster: the block K of diag(mu) + E, its transform X, and one rotation per
 // pair of a round.
@@ -234,12 +246,14 @@ constexpr size_t cluster_smem(int n) { return kClusterWarps + (size_t)n * (sizeo
 // a time in the labels 1.22 and 3.3; 32 uneven structures 20.6 -> 12.1, 7 x 5 S-matrices 1.35 -> 0.61.
 __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* __restrict__ mu,
                                                               const cf* __restrict__ E, int* lab, int* pos, int* csz,
-                                                              int* memb, cf* xc, cd* mu_out, int in_smem) {
+                                                              int* memb, cf* xc, cd* mu_out, int in_smem, int* keep,
+                                                              int first) {
   __shared__ TeamShared sh;
   __shared__ int changed;
   extern __shared__ __align__(16) unsigned char dyn_cl[];
   TeamCta t;
   const int64_t b = blockIdx.x;
+  if (keep && !keep[b]) return;
   const int64_t nn = (int64_t)n * n;
   const cd* m = mu + b * n;
   const cf* Eb = E + b * nn;
@@ -259,6 +273,28 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
   team_argmax(t, big, bi, &sh);
   big = sqrt(big);
   cluster_labels(t, n, m, in_smem ? mf : nullptr, big, lb, sz, act, &changed);
+  if (keep && first) {
+    // kUnresolved coupled eigenvalues within the FP32 solver's error of one: given up (see kUnresolved)
+    if (t.tid() == 0) changed = 0;
+    t.sync();
+    for (int i = t.tid(); i < n; i += t.size()) {
+      if (sz[i] < kUnresolved) continue;
+      int c = 0;
+      for (int j = 0; j < n; ++j) {
+        if (j == i || lb[j] != lb[i]) continue;
+        const cd d = m[j] - m[i];
+        if (!(norm2(d) < kUnresolvedTol * kUnresolvedTol * big * big)) continue;
+        const cf e = Eb[(int64_t)j * n + i];
+        c += fmaxf(fabsf(e.re), fabsf(e.im)) > kCoupledTol * (float)big;
+      }
+      if (c >= kUnresolved) changed = 1;
+    }
+    t.sync();
+    if (changed) {
+      if (t.tid() == 0) keep[b] = 0;
+      return;
+    }
+  }
   // ranks (deterministic: by index)
   for (int i = t.tid(); i < n; i += t.size()) {
     const int l = lb[i];
@@ -330,13 +366,14 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
 }
 
 int launch_clusters(int64_t batch, int n, const cd* mu, const cf* E, int* lab, int* pos, int* csz, int* memb, cf* xc,
-                    cd* mu_out, cudaStream_t s) {
+                    cd* mu_out, cudaStream_t s, int* keep = nullptr, int first = 0) {
   const int in_smem = cluster_smem(n) <= 200 * 1024 ? 1 : 0;  // (larger n: the label arrays in global memory)
   const size_t smem = in_smem ? cluster_smem(n) : kClusterWarps;
   if (smem > 40 * 1024 &&
       cudaFuncSetAttribute(k_clusters, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
     return KHP_ERR_CUDA;
-  k_clusters<<<(unsigned)batch, kClusterThreads, smem, s>>>(n, mu, E, lab, pos, csz, memb, xc, mu_out, in_smem);
+  k_clusters<<<(unsigned)batch, kClusterThreads, smem, s>>>(n, mu, E, lab, pos, csz, memb, xc, mu_out, in_smem,
+                                                             keep, first);
   count_launches(1);
   return cuda_status();
 }
@@ -361,9 +398,11 @@ __device__ __forceinline__ cf first_order(const cf* Eb, const cd* mb, int n, int
 // first-order errors in column j, and the step would not converge for clustered eigenvalues.
 __global__ void k_eig_update(int64_t boff, int n, const cd* __restrict__ mu_in, const cf* __restrict__ E, cf* F,
                              const int* __restrict__ lab, const int* __restrict__ pos, const int* __restrict__ csz,
-                             const int* __restrict__ memb, const cf* __restrict__ xc) {
+                             const int* __restrict__ memb, const cf* __restrict__ xc,
+                             const int* __restrict__ keep) {
   const int64_t nn = (int64_t)n * n;
   const int64_t b = boff + blockIdx.y;
+  if (keep && !keep[b]) return;  // (no clusters were written)
   const cf* Eb = E + b * nn;
   const cd* mb = mu_in + b * n;
   for (int rc = blockIdx.x * blockDim.x + threadIdx.x; rc < nn; rc += gridDim.x * blockDim.x) {
@@ -403,12 +442,17 @@ __device__ __forceinline__ bool rt_undefined(const double* kp, double k0, cd eps
 __global__ void __launch_bounds__(256) k_eig_check(int64_t boff, int n, const cd* __restrict__ MW,
                                                    const cd* __restrict__ W, const cd* __restrict__ mu,
                                                    const double* __restrict__ kp, const double* __restrict__ k0,
-                                                   cd epsi, double tol, int bit, int* stat) {
+                                                   cd epsi, double tol, int bit, int* stat,
+                                                   const int* __restrict__ keep) {
   __shared__ TeamShared sh;
   __shared__ double rs[8][32], wsq[8][32];
   TeamCta t;
   const int64_t b = boff + blockIdx.y;
   if (kp && rt_undefined(kp + 4 * b, k0[b], epsi)) return;
+  if (keep && !keep[b]) {
+    if (blockIdx.x == 0 && t.tid() == 0) atomicOr(stat + b, bit);
+    return;
+  }
   const int64_t nn = (int64_t)n * n;
   const cd* mb = mu + b * n;
   double big = 0.0;
@@ -1406,13 +1450,14 @@ struct EigRefine {
   float *tfA, *tfB;
   int* tferr;
   OzakiWs oz;
+  int* keep = nullptr;  // cleared for matrices that the first step gives up (null: none are)
 };
 
 int launch_eig_check(int64_t batch, int n, const cd* MW, const cd* W, const cd* mu, const double* kp, const double* k0,
-                     cd epsi, double tol, int bit, int* stat, cudaStream_t s) {
+                     cd epsi, double tol, int bit, int* stat, cudaStream_t s, const int* keep = nullptr) {
   for (int64_t o = 0; o < batch; o += 65535) {
     const unsigned nb = (unsigned)std::min<int64_t>(batch - o, 65535);
-    k_eig_check<<<dim3((n + 31) / 32, nb), 256, 0, s>>>(o, n, MW, W, mu, kp, k0, epsi, tol, bit, stat);
+    k_eig_check<<<dim3((n + 31) / 32, nb), 256, 0, s>>>(o, n, MW, W, mu, kp, k0, epsi, tol, bit, stat, keep);
     count_launches(1);
   }
   return cuda_status();
@@ -1429,7 +1474,9 @@ int refine_eigs(int64_t bm, int n, const cd* M64, cd* W64, EigRefine& r, int ste
   // the FP32 products (E = W^-1 R, W F): 3xTF32 on the tensor cores when the recursion's products
   // are (their planes are free until the recursion), else the tiled product
   auto mode_prod = [&](const cf* A, const cf* B, cf* C) -> int {
-    if (!r.tfA) return launch_gemm<float>(bm, n, n, n, one, A, n, nn, B, n, nn, zero, C, n, nn, s);
+    if (!r.tfA)
+      return launch_gemm<float>(bm, n, n, n, one, A, n, nn, B, n, nn, zero, C, n, nn, s, nullptr, nullptr, zero,
+                                r.keep);
     int st = tf32x3_split_a(bm, n, n, A, n, nn, nullptr, r.tfA, s);
     if (!st) st = tf32x3_split_b(bm, n, n, B, n, nn, nullptr, zero, r.tfB, s);
     return st ? st : tf32x3_from_planes(bm, n, n, n, r.tfA, r.tfB, one, zero, C, n, nn, r.tferr, s);
@@ -1445,10 +1492,11 @@ int refine_eigs(int64_t bm, int n, const cd* M64, cd* W64, EigRefine& r, int ste
     MX_TRY(launch_copy<float>(bm, n, n, r.W32, n, nn, r.lu32, n, nn, s));
     MX_TRY(launch_inverse_blocked<float>(bm, n, r.lu32, n, nn, r.Wi, n, nn, r.piv, r.st, s));
     MX_TRY(ozaki_zgemm(bm, n, n, n, M64, n, nn, nullptr, W64, n, nn, r.MW64, n, nn, r.oz, s, mode_step_digits()));
-    MX_PP(k_eig_residual, bm, nn, n, r.MW64, W64, r.mu, r.E32);
+    MX_PP(k_eig_residual, bm, nn, n, r.MW64, W64, r.mu, r.E32, r.keep);
     MX_TRY(mode_prod(r.Wi, r.E32, r.Z32));  // E
-    MX_TRY(launch_clusters(bm, n, r.mu, r.Z32, r.pair, r.nearest, r.csz, r.memb, r.xc, r.mu_next, s));
-    MX_PP(k_eig_update, bm, nn, n, r.mu, r.Z32, r.F32, r.pair, r.nearest, r.csz, r.memb, r.xc);
+    MX_TRY(launch_clusters(bm, n, r.mu, r.Z32, r.pair, r.nearest, r.csz, r.memb, r.xc, r.mu_next, s, r.keep,
+                           step == 0 ? 1 : 0));
+    MX_PP(k_eig_update, bm, nn, n, r.mu, r.Z32, r.F32, r.pair, r.nearest, r.csz, r.memb, r.xc, r.keep);
     MX_TRY(mode_prod(r.W32, r.F32, r.Z32));
     MX_EW(k_add_correction, bm * nn, bm * nn, W64, r.Z32, r.W32);
     std::swap(r.mu, r.mu_next);
@@ -1486,6 +1534,7 @@ RefinedWs plan_refined(Arena& a, int64_t batch, int n) {
   r.xc = a.take<cf>(b * n * kClusterMax);
   r.piv = a.take<int>(b * n);
   w.st = a.take<int>(b);
+  r.keep = a.take<int>(b);
   r.st = w.st;
   const size_t ch = std::min(b, (size_t)kOzakiMaxChunk);
   r.oz.ad_elems = ch * ozaki_a_elems(n, n);
@@ -1497,6 +1546,7 @@ RefinedWs plan_refined(Arena& a, int64_t batch, int n) {
   r.oz.eb_n = ch * n;
   r.oz.eb = a.take<int>(r.oz.eb_n);
   r.oz.err = a.take<int>(1);
+  r.oz.only = r.keep;
   r.tfA = r.tfB = nullptr;
   r.tferr = nullptr;
   if (use_tf32_products(n)) {
@@ -1817,9 +1867,11 @@ int solve_mixed(int64_t batch, int px, int py, int L, const int* kinds, const in
 // lossy maps: max|M W - W mu| / (max|mu| max|W|) up to 5e-15 at n = 18, 2e-14 at n = 98 and 1e-13 at
 // n = 242; refined: the same or less).  The FP64 QR is one CTA's chain on a pipe of 2 FMAs per clock:
 // one matrix takes 15 to 21 ms at n = 50, 60 to 77 at n = 98 and 410 to 510 at n = 242, against 3.1, 8
-// to 9 and 43 to 47 here; 64 matrices of n = 126 112 against 15 ms.  A nearly uniform symmetric map,
-// whose exactly degenerate groups are larger than a cluster, pays for both (9.4 against 12.4 ms at
-// n = 50).  Below kRefinedMinN the FP64 QR alone is as fast (n = 10: 0.7 ms each way, n = 18: 2.3
+// to 9 and 43 to 47 here; 64 matrices of n = 126 112 against 15 ms.  A matrix that misses the test pays for
+// both, so a hopeless one is given up before its first step (kUnresolved) and the FP64 eigensolver's Z goes
+// through the rotation log: nearly uniform maps at normal incidence, FP64 eigensolver alone before / with all
+// steps before it / so: n = 18 1.64 / 2.70 / 1.65 ms, 50 9.0 / 11.2 / 7.2, 98 37.9 / 40.3 / 28.6, 242 271 / 279 /
+// 193; 304 of n = 98 51 / 91 / 49.  Below kRefinedMinN the FP64 QR alone is as fast (n = 10: 0.7 ms each way, n = 18: 2.3
 // against 1.0).
 constexpr int kRefinedMinN = 12;
 constexpr int kRefinedMaxN = 4096;  // the digit products' limit
@@ -1887,6 +1939,7 @@ int launch_geev_refined(int64_t batch, int n, cd* M, cd* W, cd* lam, int* info, 
     cd* Mo = M + o * nn;
     cd* Wo = W + o * nn;
     if (cudaMemsetAsync(w.st, 0, sizeof(int) * bm, s) != cudaSuccess) return KHP_ERR_CUDA;
+    if (cudaMemsetAsync(r.keep, 1, sizeof(int) * bm, s) != cudaSuccess) return KHP_ERR_CUDA;  // (any nonzero)
     MX_EW(k_round, bm * nn, bm * nn, Mo, w.M32);
     MX_TRY(launch_geev<float>(bm, n, w.M32, n, nn, r.Z32, r.W32, n, nn, w.lam32, n, w.st, s, r.MW64,
                               (int64_t)(nn * sizeof(cd)) / 32 * 32));
@@ -1894,13 +1947,16 @@ int launch_geev_refined(int64_t batch, int n, cd* M, cd* W, cd* lam, int* info, 
     MX_TRY(ozaki_zgemm(bm, n, n, n, Mo, n, nn, nullptr, Wo, n, nn, r.MW64, n, nn, r.oz, s));
     if (cudaMemcpyAsync(act + o, w.st, sizeof(int) * bm, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       return KHP_ERR_CUDA;
-    MX_TRY(launch_eig_check(bm, n, r.MW64, Wo, r.mu, nullptr, nullptr, mk(0.0), kRefinedTolPerN * n, 1, act + o, s));
+    MX_TRY(launch_eig_check(bm, n, r.MW64, Wo, r.mu, nullptr, nullptr, mk(0.0), kRefinedTolPerN * n, 1, act + o, s,
+                            r.keep));
     if (cudaMemcpyAsync(lam + o * n, r.mu, sizeof(cd) * bm * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       return KHP_ERR_CUDA;
   }
   MX_TRY(launch_normalize_cols<double>(batch, n, W, n, nn, W, n, nn, s));
-  return launch_geev<double>(batch, n, M, n, nn, reinterpret_cast<cd*>(base), W, n, nn, lam, n, info, s, nullptr, 0,
-                             act);
+  // (what is left of the scratch beside Z holds the QR's rotation logs)
+  const size_t zp = (z + 255) & ~size_t(255), left = ws_bytes - mask > zp ? ws_bytes - mask - zp : 0;
+  return launch_geev<double>(batch, n, M, n, nn, reinterpret_cast<cd*>(base), W, n, nn, lam, n, info, s, base + zp,
+                             (int64_t)(left / batch / 32 * 32), act);
 }
 
 int mixed_modes_in_workspace(int64_t batch, int nh, int L, const int* kinds, const int* maps, const void* ws,

@@ -110,11 +110,12 @@ __device__ __forceinline__ void put_digits7(double x, int e, bf16* out, int64_t 
 template <int ND, typename TI>
 __global__ void k_tc_split_a(int64_t batch, int m, int k, const cplx<TI>* __restrict__ A, int64_t lda, int64_t bsA,
                              const int* __restrict__ aidx, int Mp, int K2p, bf16* __restrict__ Ad,
-                             int* __restrict__ ea) {
+                             int* __restrict__ ea, const int* __restrict__ only) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < batch * Mp; w += nwarps) {
     const int64_t b = w / Mp;
+    if (only && !only[b]) continue;
     const int r = (int)(w % Mp);
     const bool live = r < m;
     const cplx<TI>* row = A + (aidx ? (int64_t)aidx[b] : b) * bsA + (int64_t)r * lda;
@@ -139,9 +140,10 @@ __global__ void k_tc_split_a(int64_t batch, int m, int k, const cplx<TI>* __rest
 // Column exponents of B, thread per (problem, column).
 template <typename TI>
 __global__ void k_tc_col_exp(int64_t batch, int k, int n, const cplx<TI>* __restrict__ B, int64_t ldb, int64_t bsB,
-                             const int* __restrict__ bidx, int* __restrict__ eb) {
+                             const int* __restrict__ bidx, int* __restrict__ eb, const int* __restrict__ only) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < batch * n; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = e / n;
+    if (only && !only[b]) continue;
     const int c = (int)(e % n);
     const cplx<TI>* col = B + (bidx ? (int64_t)bidx[b] : b) * bsB + c;
     int bm = 0;
@@ -159,9 +161,11 @@ __global__ void k_tc_col_exp(int64_t batch, int k, int n, const cplx<TI>* __rest
 template <int ND, typename TI>
 __global__ void __launch_bounds__(256) k_tc_split_b(int k, int n, const cplx<TI>* __restrict__ B, int64_t ldb,
                                                     int64_t bsB, const int* __restrict__ bidx, int N2p, int K2p,
-                                                    const int* __restrict__ eb, bf16* __restrict__ Bd) {
+                                                    const int* __restrict__ eb, bf16* __restrict__ Bd,
+                                                    const int* __restrict__ only) {
   __shared__ double xs[32][33];
   const int64_t b = blockIdx.z;
+  if (only && !only[b]) return;
   const int j0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const cplx<TI>* Bb = B + (bidx ? (int64_t)bidx[b] : b) * bsB;
@@ -278,7 +282,8 @@ template <int ND, typename TO>
 __global__ void __launch_bounds__(kThreads, 1)
     k_tc_digits(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int m, int n, int Mp,
                 int K2p, const int* __restrict__ ea, const int* __restrict__ eb, cplx<TO>* C, int64_t ldc, int64_t bsC,
-                cplx<TO> alpha, cplx<TO> beta, int use_beta, int* err) {
+                cplx<TO> alpha, cplx<TO> beta, int use_beta, int* err, const int* __restrict__ only) {
+  if (only && !only[blockIdx.z]) return;  // (the whole CTA, before it holds anything)
   constexpr int NT = TcCfg<ND>::NT;
   constexpr uint32_t kTileB = NT * 128;  // one digit's B tile (bytes)
   constexpr uint32_t kTileA = kM * 128;
@@ -736,23 +741,25 @@ int tc_product(int64_t batch, int m, int n, int k, const cplx<TI>* A, int64_t ld
     bf16* Adg = static_cast<bf16*>(w.ad);
     bf16* Bdg = static_cast<bf16*>(w.bd);
     k_tc_split_a<ND, TI><<<grid_of(nb * Mp * 32, 256), 256, 0, s>>>(
-        nb, m, k, aidx ? A : A + off * bsA, lda, bsA, aidx ? aidx + off : nullptr, Mp, K2p, Adg, w.ea);
+        nb, m, k, aidx ? A : A + off * bsA, lda, bsA, aidx ? aidx + off : nullptr, Mp, K2p, Adg, w.ea,
+        w.only ? w.only + off : nullptr);
     k_tc_col_exp<TI><<<grid_of(nb * n, 128), 128, 0, s>>>(nb, k, n, bidx ? B : B + off * bsB, ldb, bsB,
-                                                         bidx ? bidx + off : nullptr, w.eb);
+                                                         bidx ? bidx + off : nullptr, w.eb,
+                                                         w.only ? w.only + off : nullptr);
     count_launches(2);
     for (int64_t o2 = 0; o2 < nb; o2 += 65535) {
       const unsigned z = (unsigned)std::min<int64_t>(nb - o2, 65535);
       const int64_t bo = off + o2;
       k_tc_split_b<ND, TI><<<dim3(N2p / 32, K2p / 32, z), dim3(32, 8), 0, s>>>(
           k, n, bidx ? B : B + bo * bsB, ldb, bsB, bidx ? bidx + bo : nullptr, N2p, K2p, w.eb + o2 * n,
-          Bdg + o2 * per_b);
+          Bdg + o2 * per_b, w.only ? w.only + bo : nullptr);
       CUtensorMap tmA, tmB;
       if (!encode_digits_map(&tmA, Adg + o2 * per_a, K2p, Mp, (int64_t)z * ND, kM) ||
           !encode_digits_map(&tmB, Bdg + o2 * per_b, K2p, N2p, (int64_t)z * ND, NT))
         return KHP_ERR_CUDA;
       k_tc_digits<ND, TO><<<dim3(N2p / NT, Mp / kM, z), kThreads, smem, s>>>(
           tmA, tmB, m, n, Mp, K2p, w.ea + o2 * Mp, w.eb + o2 * n, C + bo * bsC, ldc, bsC, alpha, beta,
-          use_beta ? 1 : 0, w.err);
+          use_beta ? 1 : 0, w.err, w.only ? w.only + bo : nullptr);
       count_launches(2);
     }
     const int st = cuda_status();
