@@ -51,8 +51,8 @@ const char* khp_status_string(int code);
 /*
  * Launch tuning, process-wide (no counterpart in the reference).  param KHP_TUNE_EIG_THREADS:
  * threads per CTA of the batched eigensolver (Hessenberg reduction and QR) for matrices of
- * size n (1 <= n <= 4096): a multiple of 32 up to 256, or 0 for the default (256; the FP32 QR's by
- * size and batch, which also holds for batches of at most one matrix per SM).  The results
+ * size n (1 <= n <= 4096): a multiple of 32 up to 256 (the FP32 QR takes at least 64), or 0 for the
+ * library's choice by precision, size and batch.  The results
  * do not depend on it; the speed does (small matrices leave a 256-thread team mostly idle).  Set
  * it before the launches it should affect (it is read when a call enqueues its kernels).
  * khepri_gb300.autotune measures the choices and writes the table the Python API applies.

@@ -30,6 +30,7 @@ import torch
 from . import _capi
 
 TUNING_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning.json")
+SMS = 152
 _table = None
 
 
@@ -54,11 +55,14 @@ class tuned_team:
     """Context manager: the tuned eigensolver team size for matrices of size n inside, the default
     after.  The team size is tuned together with the matrices per call, so it applies only to
     calls that also take ``chunk_for``'s chunk (a 128-thread team that wins at 912 matrices per
-    call loses at 456)."""
+    call loses at 456), and not to their last ones of at most a matrix per SM (``matrices``), where the
+    library's larger teams are faster."""
 
-    def __init__(self, n):
+    def __init__(self, n, matrices=None):
         self.n = int(n)
         self.threads = int(table().get(self.n, {}).get("eig_threads", 0))
+        if matrices is not None and matrices <= SMS:
+            self.threads = 0
 
     def __enter__(self):
         if self.threads:

@@ -719,7 +719,8 @@ def solve_structures(structures, wavelengths, kp, which=None, te=1.0, tm=0.0, la
             prob = engine.Problems.make(wl[idx], kpa[idx], te[idx], tm[idx], dev)
             status = torch.zeros(B, dtype=torch.int32, device=dev)
             # the autotuned chunk comes with its tuned eigensolver team size
-            with (autotune.tuned_team(struct_k.n) if chunk is None else contextlib.nullcontext()):
+            mats = B * len({m for kind, m in zip(plan.kinds, plan.maps) if kind == 1})
+            with (autotune.tuned_team(struct_k.n, mats) if chunk is None else contextlib.nullcontext()):
                 if both_pols:
                     tt, tmm = both_pol_weights(B, dev)
                     r, t, fix = solve_chunk_gamma(struct_k, plan, prob, status, epsi, epse, tt, tmm, prec, refine,

@@ -6,12 +6,12 @@
 #include "khp_dense.cuh"
 #include "khp_hqr.cuh"
 #include "khp_launch.h"
+#include "khp_teams.h"
 
 namespace khp {
 
 namespace {
 
-constexpr int kTeamThreads = 256;
 constexpr int64_t kMaxGridY = 65535;
 
 // Threads per eigensolver CTA by matrix size (khp_tune; 0 = kTeamThreads).  Small matrices leave
@@ -19,11 +19,7 @@ constexpr int64_t kMaxGridY = 65535;
 constexpr int kTuneMaxN = 4096;
 int g_eig_threads[kTuneMaxN + 1] = {0};
 
-bool eig_tuned(int n) { return n <= kTuneMaxN && g_eig_threads[n] > 0; }
-int eig_threads(int n) {
-  const int v = n <= kTuneMaxN ? g_eig_threads[n] : 0;
-  return v > 0 ? v : kTeamThreads;
-}
+int eig_tuned(int n) { return n <= kTuneMaxN ? g_eig_threads[n] : 0; }
 
 }  // namespace
 
@@ -1013,12 +1009,7 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(k_gehrd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return KHP_ERR_CUDA;
-  // (FP64: smaller teams for small matrices, whose barriers and reductions are most of a step; one n = 18
-  // 1.64 ms with 256 threads, 1.55 with 64; n = 50 8.96, 8.76 with 128; n = 98 the fastest with 256)
-  const int threads = sizeof(T) == 8 && !eig_tuned(n) ? (n <= 32   ? 64
-                                                         : n <= 64 ? 128
-                                                                   : kTeamThreads)
-                                                      : eig_threads(n);
+  const int threads = eig_team(sizeof(T) == 8, n, eig_tuned(n));
   // the blocked reduction keeps full 256-thread teams (its panel updates are parallel work; three
   // teams per SM already cover the SM), whatever team size suits the QR's serial window chase
   const int gthreads = blocked ? kTeamThreads : threads;
@@ -1040,21 +1031,7 @@ int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx
   if (logbuf && log_fits && log_bytes % 32 == 0 && reinterpret_cast<uintptr_t>(logbuf) % 32 == 0 &&
       hqr_log_view<T>(logbuf, log_bytes, n).cap_rot >= n - 1)
     lg = static_cast<unsigned char*>(logbuf);
-  // FP32: a warp for the chase, the others for the strips.  While a matrix has an SM to itself more threads
-  // than strips shorten their way to and from H (one n = 242: 256 threads 11.2 ms, 288 10.5, 352 9.4, 480
-  // 9.3, 544 with the warps on the chase's scheduler idle 9.0, 480 so 9.2; n = 162: 4.87, 4.83, 4.09, 4.15, 3.94,
-  // 4.21; n = 50: 557, 561, 542, 547, 555, 558 us).  Up to two matrices per SM two CTAs
-  // fit with 256 (304 of n = 98: 192 threads 2.67 ms, 256 2.41, 352 3.44).  Beyond, three of 192 where their
-  // shared memory fits (456 of n = 98: 192 threads 3.22, 256 4.48; of n = 150: 7.17, 8.87), else two of 288
-  // (456 of n = 162: 192 threads 13.8, 256 12.2, 288 11.0; of n = 242: 32.1, 29.5, 25.3).  Small matrices: 512
-  // of n = 18 with 128 threads 284 us, 160 270, 192 368.
-  const int sthreads = sizeof(T) == 8 || !lg           ? threads
-                       : eig_tuned(n) && batch > 152   ? std::max(64, threads)
-                       : n <= 32                       ? 160
-                       : batch <= 152                  ? (n <= 64 ? 352 : 544)
-                       : batch <= 2 * 152              ? kTeamThreads
-                       : n <= 150                      ? 192
-                                                       : kTeamThreads + 32;
+  const int sthreads = sizeof(T) == 8 || !lg ? threads : chase_team(n, batch, eig_tuned(n));
   // (FP64 teams end at 256, so that two share an SM: with the registers that 288 threads may take only one
   // fits, and 304 scattering eigenproblems of N = 100 took 154 instead of 94 ms, of N = 36 22 instead of 13)
   auto schur = k_geev_schur<T, sizeof(T) == 8 ? kTeamThreads : kTeamThreads + 32>;
