@@ -26,10 +26,10 @@ KHP_HD void label_min(int* p, int v) {
 }
 
 // Labels of the n eigenvalues m, big = max|m|: lb[i] becomes the smallest index of i's component, so
-// lb[lb[i]] == lb[i], and sz[i] the component's size.  mf: the eigenvalues rounded to FP32, or null; act: n
-// ints of scratch; changed: one int shared by the team.  Distances are taken in FP32 where that decides
-// as FP64 would (mf given).
-template <class Team>
+// lb[lb[i]] == lb[i], and sz[i] the component's size.  act: n ints of scratch; changed: one int shared by the
+// team.  kRounded: mf holds the eigenvalues rounded to FP32, and distances are taken in FP32 where that
+// decides as FP64 would.
+template <bool kRounded, class Team>
 KHP_HD void cluster_labels(const Team& t, int n, const cplx<double>* m, const cplx<float>* mf, double big, int* lb,
                            int* sz, int* act, int* changed) {
   double tol = kClusterTol * big;
@@ -66,7 +66,7 @@ KHP_HD void cluster_labels(const Team& t, int n, const cplx<double>* m, const cp
         if (!act[i]) continue;
         const int old = lb[i];
         int best = old;
-        if (mf && scaled) {  // eight columns' loads at a time (a label read a little early is only older)
+        if (kRounded && scaled) {  // eight columns' loads at a time (a label read a little early is only older)
           const cplx<float> mi = mf[i];
           for (int j0 = 0; j0 < n; j0 += 8) {
             cplx<float> q[8];

@@ -272,7 +272,12 @@ __global__ void __launch_bounds__(kClusterThreads) k_clusters(int n, const cd* _
   }
   team_argmax(t, big, bi, &sh);
   big = sqrt(big);
-  cluster_labels(t, n, m, in_smem ? mf : nullptr, big, lb, sz, act, &changed);
+  if (in_smem) {  // (arrays known to lie in shared memory)
+    int* l = reinterpret_cast<int*>(mf + n);
+    cluster_labels<true>(t, n, m, mf, big, l, l + n, l + 2 * n, &changed);
+  } else {
+    cluster_labels<false>(t, n, m, mf, big, lb, sz, act, &changed);
+  }
   if (keep && first) {
     // kUnresolved coupled eigenvalues within the FP32 solver's error of one: given up (see kUnresolved)
     if (t.tid() == 0) changed = 0;

@@ -18,5 +18,8 @@ extern "C" void host_cluster_labels(int n, const double* mu, int fp32, int* lb, 
     lb[i] = i;
   }
   int changed = 0;
-  cluster_labels(TeamSerial(), n, m, fp32 ? mf.data() : nullptr, std::sqrt(big), lb, sz, act.data(), &changed);
+  if (fp32)
+    cluster_labels<true>(TeamSerial(), n, m, mf.data(), std::sqrt(big), lb, sz, act.data(), &changed);
+  else
+    cluster_labels<false>(TeamSerial(), n, m, mf.data(), std::sqrt(big), lb, sz, act.data(), &changed);
 }
