@@ -6,6 +6,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "khepri_gb300.h"
 #include "khp_core.cuh"
@@ -306,9 +307,14 @@ bool gehrd_cluster_fits(int64_t batch, int n) {
   // SM (k_gehrd; n = 338, 304 matrices: 46 ms against 52; n = 578, 64: 207 against 61)
   if (C == 8 && hess_smem(n, C) > 74 * 1024 && batch > 256) return false;
   if (C < 16) return C > 0;
-  // a cluster of 16 is beyond the portable size: ask whether this device can hold one
-  static int can16 = -1;
-  if (can16 < 0) {
+  // a cluster of 16 is beyond the portable size: ask whether the device can hold one (once per device; callers
+  // of several threads may all ask, and get the same answer)
+  constexpr int kDevices = 64;
+  static std::atomic<int> can16[kDevices];  // 0: not asked, 1: no, 2: yes
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return false;
+  int can = can16[dev].load(std::memory_order_relaxed);
+  if (can == 0) {
     int ok = 0;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[1];
@@ -326,9 +332,10 @@ bool gehrd_cluster_fits(int64_t batch, int n) {
       cudaGetLastError();
       ok = 0;
     }
-    can16 = ok > 0 ? 1 : 0;
+    can = ok > 0 ? 2 : 1;
+    can16[dev].store(can, std::memory_order_relaxed);
   }
-  return can16 == 1;
+  return can == 2;
 }
 
 int launch_gehrd_cluster(int64_t batch, int n, cplx<float>* A, int64_t lda, int64_t bsA, cplx<float>* V, int64_t ldv,
