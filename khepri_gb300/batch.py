@@ -828,9 +828,9 @@ def solve_structures_grad(structures, wavelengths, kp, which=None, dR=None, dT=N
                 for k, d in zip(sel, deps):
                     sid, slot = maps[k]
                     _, layers, stack = structures[sid]
-                    for l, name in enumerate(stack):
-                        if plan.kinds[l] == 1 and plan.maps[l] == slot:
-                            grads[sid][name] = grads[sid].get(name, 0) + d
+                    # d is the slot's total over the stack: once per layer name, however often it stands there
+                    for name in {nm for l, nm in enumerate(stack) if plan.kinds[l] == 1 and plan.maps[l] == slot}:
+                        grads[sid][name] = grads[sid].get(name, 0) + d
     if strict and st_all.any():
         bad = int(np.flatnonzero(st_all)[0])
         raise _capi.KhpError(f"problem {bad}: {_capi.decode_status(int(st_all[bad]))}")
