@@ -89,14 +89,12 @@ KHP_HD void cluster_labels(const Team& t, int n, const cplx<double>* m, const cp
           for (int j = 0; j < n; ++j)
             if (act[j] && lb[j] < best && close64(i, j)) best = lb[j];
         }
-        int next = lb[best];
-        while (next < best) {
-          best = next;
-          next = lb[best];
-        }
+        const int next = lb[best];
+        if (next < best) best = next;
         if (best < old) {
-          label_min(lb + i, best);
-          label_min(lb + old, best);
+          // (a label passed to i in between may be lost here: another round follows)
+          lb[i] = best;
+          if (old != i) label_min(lb + old, best);
           *changed = 1;
         }
       }

@@ -30,12 +30,13 @@ __device__ __forceinline__ unsigned pivot_key(cplx<double> v) {
   if (!(x == x)) return 0u;
   return x == 0.0 ? 1u : max((unsigned)__double2hiint(x), 1u) + 1u;
 }
-// Status of a step from its best candidate's key.  An infinite pivot would eliminate with a reciprocal of
-// 0 and leave a finite "inverse" of a matrix that has none.
+// Status of a step from its best candidate's key, 0 for a nonzero finite pivot.  (An infinite one would
+// eliminate with a reciprocal of 0 and leave a finite "inverse" of a matrix that has none.)
 template <typename T>
 __device__ __forceinline__ int pivot_status(unsigned best) {
   constexpr unsigned kInf = (sizeof(T) == 4 ? 0x7f800000u : 0x7ff00000u) + 1u;
-  return best == 1u ? KHP_BIT_SINGULAR : best == 0u || best >= kInf ? KHP_BIT_NONFINITE : 0;
+  if (best - 2u < kInf - 2u) return 0;  // (one comparison on the elimination's chain)
+  return best == 1u ? KHP_BIT_SINGULAR : KHP_BIT_NONFINITE;
 }
 
 // 1/p for a pivot (nonzero): conj(p)/|p|^2 with p scaled by a power of two to a modulus of 1 to 2^1.5, one
@@ -118,12 +119,12 @@ __global__ void __launch_bounds__(32 * NW) k_inv_reg(int n, const cplx<float>* _
     pv.re = __shfl_sync(0xffffffffu, pv.re, p & 31);
     pv.im = __shfl_sync(0xffffffffu, pv.im, p & 31);
     const bool ok = best > 1u;  // 1: every candidate is 0; 0: every candidate is NaN
-    st |= pivot_status<float>(best);
     if (lane == 0) {
       pinv_s[buf] = ok ? pivot_recip(pv) : mk(0.f);
       pcol_s[buf] = ok ? p : ~p;  // ~p: the column is spent but nothing is eliminated
       pcol[k] = p;
       kinv[p] = k;
+      st |= pivot_status<float>(best);
     }
   };
   if (warp == 0) {
@@ -219,7 +220,6 @@ __global__ void __launch_bounds__(32 * NW) k_inv_reg(int n, const cplx<float>* _
         if (lane + 32 * i < n) out[kinv[lane + 32 * i]] = a[i][j];
     }
   }
-  for (int o = 16; o > 0; o >>= 1) st |= __shfl_xor_sync(0xffffffffu, st, o);
   if (lane == 0 && st) atomicOr(info + blockIdx.x, st);
 }
 
