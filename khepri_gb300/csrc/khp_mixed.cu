@@ -1416,9 +1416,10 @@ GradPlan plan_grad(Arena& a, int64_t batch, int nh, int L, int64_t nmaps) {
   return g;
 }
 
-// Threads of the per-problem stack kernels: 512 while a problem has an SM to itself, else 256 (912
-// problems of n = 98 1.4 against 1.7 ms a call with 512).
-int stack_threads(int64_t batch) { return batch <= 2 * 152 ? 32 * kPartWarps : 256; }
+// Threads of the per-problem stack kernels: 512 while a problem has an SM to itself, else 256 (five layers, 304
+// problems of n = 50 a call 8.08 ms with 512, 7.55 with 256, of n = 242 105.3 and 105.0; 912 of n = 98 in
+// these kernels 1.7 and 1.4).
+int stack_threads(int64_t batch) { return batch <= 152 ? 32 * kPartWarps : 256; }
 
 #define MX_TRY(x)        \
   do {                   \
