@@ -111,6 +111,8 @@ int khp_structure_prep(int64_t nmaps, int32_t nh, const double* conv, const doub
  *   map_index: int32 [batch] structure of each problem (into conv/hx/hy, [nmaps][nh][nh]);
  *   kp: complex [batch][2] in-plane wavevector (absolute); k0: real [batch] = 2 pi / wavelength;
  *   W, V: complex [batch][n][n];  lam: complex [batch][n];  status: int32 [batch].
+ *   Workspace: 48 bytes per entry of the n x n matrices, or up to 2 GiB where that lets the eigensolver
+ *   take more of them at a time.
  */
 size_t khp_layer_modes_workspace(int64_t batch, int32_t nh);
 int khp_layer_modes(int64_t batch, int32_t nh, const int32_t* map_index, const double* conv, const double* hx,
@@ -171,6 +173,9 @@ int khp_star_product(int64_t batch, int32_t n, const double* SA, int64_t sa_stri
  *   conv, hx, hy: device complex [nmaps][nh][nh] from khp_convmat / khp_structure_prep;
  *   kp: complex [batch][2]; k0: [batch]; te, tm: complex [batch][npol] (npol polarisations
  *   share one recursion);  R, T: real [batch][npol].
+ *   Workspace: the recursion's arrays (16 bytes per entry of n x n: 5 per distinct map, 2 per patterned
+ *   layer, 1 per other layer, 8 more), of which the eigensolver uses those not yet in use, or up to 2 GiB
+ *   where that lets it take more matrices at a time.
  */
 size_t khp_solve_batched_workspace(int64_t batch, int32_t nh, int32_t nlayers, const int32_t* layer_kind,
                                    const int32_t* layer_map);
@@ -497,9 +502,11 @@ int khp_inverse(int64_t batch, int32_t n, int32_t precision, void* A, int64_t a_
 
 /*
  * The same inverse by Gauss-Jordan elimination with partial pivoting (the form the mixed-precision
- * solve uses: one launch per call up to n = 128 in FP32, two launches per 32 rows otherwise).
- * Arguments, status and scratch as khp_inverse; A is overwritten with intermediate values and
- * must not overlap Ainv.
+ * solve uses).  FP32 up to n = 128: one launch; up to n = 1024 two launches per panel of 32 rows (FP32;
+ * 24 from n = 767 and 16 from n = 1013, as a panel lies in shared memory) or 8 rows (FP64), the first
+ * panel halved where their number is even; beyond, the blocked LU of khp_inverse.  No pivot left but 0
+ * sets SINGULAR; a NaN or an infinity in the matrix sets NONFINITE.  Arguments, status and scratch as
+ * khp_inverse; A is overwritten with intermediate values and must not overlap Ainv.
  */
 int khp_inverse_gj(int64_t batch, int32_t n, int32_t precision, void* A, int64_t a_stride, void* Ainv,
                    int64_t inv_stride, int32_t* status, void* workspace, size_t ws_bytes, void* stream);

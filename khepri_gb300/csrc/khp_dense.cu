@@ -14,8 +14,7 @@ namespace {
 
 constexpr int64_t kMaxGridY = 65535;
 
-// Threads per eigensolver CTA by matrix size (khp_tune; 0 = kTeamThreads).  Small matrices leave
-// most of a 256-thread team idle, and smaller teams let more matrices share an SM.
+// Threads per eigensolver CTA by matrix size that the caller set (khp_tune; 0: none, khp_teams.h decides).
 constexpr int kTuneMaxN = 4096;
 int g_eig_threads[kTuneMaxN + 1] = {0};
 

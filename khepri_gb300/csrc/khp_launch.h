@@ -29,8 +29,9 @@ int launch_gemm(int64_t batch, int n, int m, int k, cplx<T> alpha, const cplx<T>
 
 // Eigen-decomposition A W = W diag(lam); A destroyed; Z: batch x n x n scratch (ld n).
 // logbuf (optional, log_bytes per matrix, both multiples of 32): scratch for the QR's rotation
-// log, which defers the updates of Z (used when it holds at least one full sweep, and without
-// `only`).  only (optional, device int[batch]): matrices with only[b] == 0 are left alone.
+// log, which defers the updates of Z (used when it holds at least one full sweep; FP64: from n = 33 up to
+// where 32 rows of Z fit in shared memory, about 420).  only (optional, device int[batch]): matrices with
+// only[b] == 0 are left alone.
 template <typename T>
 int launch_geev(int64_t batch, int n, cplx<T>* A, int64_t lda, int64_t bsA, cplx<T>* Z, cplx<T>* W, int64_t ldw,
                 int64_t bsW, cplx<T>* lam, int64_t bsLam, int* info, cudaStream_t s, void* logbuf = nullptr,

@@ -13,7 +13,7 @@
 //      exact digit splitting (ozaki_zgemm), FP64-accurate;
 //   2. the reflection-matrix recursion of khp_solve_batched on the FP32-rounded refined modes,
 //      keeping every factor it makes (the explicit inverses, rho, Gamma at every gap, Gamma M^-1),
-//      with every O(n^3) step a blocked LU / inverse or a tiled product;
+//      with every O(n^3) step a Gauss-Jordan inverse or a tiled product;
 //   3. iterative refinement of the interface-continuity system of the whole stack (the
 //      equations the reference's S-matrix chain encodes, crystal.py:180-206 / layer.py:35-60),
 //      for the two source columns: residual in FP64 with the refined FP64 modes and the FP64
@@ -44,7 +44,7 @@ constexpr int kMaxLayers = 16;
 constexpr int kEigSteps = 3;
 // Refinement rounds beyond the requested ones, run only for problems not yet converged.
 constexpr int kExtraRounds = 12;
-// Largest refine_iters the entry points accept (every round is one residual and one sweep launch).
+// Largest refine_iters the entry points accept.
 constexpr int kMaxRefine = 64;
 
 // ------------------------------------------------------------------------------------------
